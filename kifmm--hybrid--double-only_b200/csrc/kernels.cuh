@@ -11,6 +11,7 @@
 //                (see spec_index)             double2 or float2 (mixed)
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -1667,34 +1668,72 @@ __global__ void error_fold_kernel(int* error) {
   if (error[0]) error[1] = 1;
 }
 
-// Plain direct sum (ulist__direct_evaluation) over SoA device arrays.
-__global__ void __launch_bounds__(128) direct_fp64_kernel(int nt, const double* tx,
-                                                          const double* ty, const double* tz,
-                                                          double* pot, int ns, const double* sx,
-                                                          const double* sy, const double* sz,
-                                                          const double* den) {
-  __shared__ double4 stage[256];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double x = 0, y = 0, z = 0, acc = 0;
+// Direct sum (ulist__direct_evaluation) over SoA device arrays, any coordinates.
+// Bound by the FP64 pipe (12 operations a pair, pair_rsqrt).  A warp takes 32
+// targets, one per lane, and every (kSplit x cluster size)-th chunk of 32 sources,
+// staged in its slice of shared memory and read back as broadcasts, the next
+// chunk prefetched into registers; a CTA's 16 warps are 16 / kSplit target tiles
+// times kSplit shares of the sources.  The shares are added in a fixed order, a
+// CTA's through shared memory and a cluster's through distributed shared memory,
+// so there is no scratch array, no atomic and one launch.
+constexpr int kDirectWarps = 16;
+constexpr int kDirectCluster = 8;
+
+template <int kSplit>
+__global__ void __launch_bounds__(32 * kDirectWarps, 2)
+direct_fp64_kernel(int nt, const double* tx, const double* ty, const double* tz, double* pot,
+                   int ns, const double* sx, const double* sy, const double* sz,
+                   const double* den) {
+  __shared__ double4 stage[kDirectWarps][32];
+  __shared__ double part[kDirectWarps][32];
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int nrank = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tile = (int)(blockIdx.x / nrank) * (kDirectWarps / kSplit) + warp / kSplit;
+  const long long i = (long long)tile * 32 + lane;
+  double x[1] = {0.0}, y[1] = {0.0}, z[1] = {0.0}, acc[1] = {0.0};
   if (i < nt) {
-    x = tx[i];
-    y = ty[i];
-    z = tz[i];
+    x[0] = tx[i];
+    y[0] = ty[i];
+    z[0] = tz[i];
   }
-  for (int b = 0; b < ns; b += 256) {
-    const int m = min(256, ns - b);
-    for (int k = threadIdx.x; k < m; k += blockDim.x)
-      stage[k] = make_double4(sx[b + k], sy[b + k], sz[b + k], den[b + k]);
-    __syncthreads();
-    for (int j = 0; j < m; ++j) {
-      const double4 s = stage[j];
-      const double dx = x - s.x, dy = y - s.y, dz = z - s.z;
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      acc = fma(s.w, r2 > 0.0 ? rsqrt(r2) : 0.0, acc);
+  const int nchunks = (int)(((long long)ns + 31) / 32), step = kSplit * nrank;
+  double4 s = make_double4(0.0, 0.0, 0.0, 0.0);
+  auto fetch = [&](int c) {
+    const int b = 32 * c;
+    if (c < nchunks && lane < ns - b)
+      s = make_double4(sx[b + lane], sy[b + lane], sz[b + lane], den[b + lane]);
+  };
+  if ((long long)tile * 32 < nt) {  // warp-uniform
+    int c = rank * kSplit + warp % kSplit;
+    fetch(c);
+    for (; c < nchunks; c += step) {
+      stage[warp][lane] = s;
+      __syncwarp();
+      fetch(c + step);
+      pairs_fp64<1, true>(x, y, z, acc, stage[warp], min(32, ns - 32 * c));
+      __syncwarp();
     }
-    __syncthreads();
   }
-  if (i < nt) pot[i] += kOOFP * acc;
+  if constexpr (kSplit == 1) {
+    if (i < nt) pot[i] += kOOFP * acc[0];
+  } else {
+    part[warp][lane] = acc[0];
+    __syncthreads();
+    if (warp % kSplit == 0) {
+      double sum = part[warp][lane];
+#pragma unroll
+      for (int w = 1; w < kSplit; ++w) sum += part[warp + w][lane];
+      part[warp][lane] = sum;
+    }
+    cluster.sync();
+    if (rank == 0 && warp % kSplit == 0 && i < nt) {
+      double sum = 0.0;
+      for (int r = 0; r < nrank; ++r) sum += cluster.map_shared_rank(&part[warp][lane], r)[0];
+      pot[i] += kOOFP * sum;
+    }
+    cluster.sync();  // the other blocks' shared memory stays until it is read
+  }
 }
 
 }  // namespace kfmm

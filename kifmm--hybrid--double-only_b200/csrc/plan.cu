@@ -1825,9 +1825,34 @@ kfmm_status kfmm_direct_evaluation(int nt, const double* tx, const double* ty, c
     return KFMM_ERR_INVALID;
   }
   if (nt == 0 || ns == 0) return KFMM_OK;
-  direct_fp64_kernel<<<(nt + 127) / 128, 128, 0, S(stream)>>>(nt, tx, ty, tz, pot, ns, sx, sy, sz,
-                                                              den);
-  KF_CHECK_LAUNCH("direct_fp64_kernel");
+  int dev = 0, sms = 0;
+  KF_CUDA(cudaGetDevice(&dev));
+  KF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  // The sources are split so that every SM holds its 32 warps (two blocks), as
+  // long as each share keeps four chunks of 32 sources: a share's start and its
+  // part of the reduction cost about as much as one chunk.
+  const long long tiles = ((long long)nt + 31) / 32, chunks = ((long long)ns + 31) / 32;
+  int split = 1;
+  for (int s : {4, kDirectWarps, kDirectWarps * kDirectCluster})
+    if (tiles * split < 2ll * kDirectWarps * sms && chunks >= 4ll * s) split = s;
+  const int warps = std::min(split, kDirectWarps), ranks = split / warps;
+  cudaLaunchConfig_t cfg = {};
+  const long long per = kDirectWarps / warps;
+  cfg.gridDim = dim3((unsigned)((tiles + per - 1) / per * ranks));
+  cfg.blockDim = dim3(32 * kDirectWarps);
+  cfg.stream = S(stream);
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ranks;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  auto launch = [&](auto kern) {
+    return cudaLaunchKernelEx(&cfg, kern, nt, tx, ty, tz, pot, ns, sx, sy, sz, den);
+  };
+  KF_CUDA(warps == 1 ? launch(direct_fp64_kernel<1>)
+                     : warps == 4 ? launch(direct_fp64_kernel<4>)
+                                  : launch(direct_fp64_kernel<kDirectWarps>));
   return KFMM_OK;
 }
 
