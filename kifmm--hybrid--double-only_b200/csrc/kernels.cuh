@@ -28,25 +28,31 @@ __device__ __forceinline__ unsigned smem_addr(const void* p) {
 // ---------------------------------------------------------------------------
 // P2P engine.  A job evaluates one set of targets against a list of source
 // sets ("entries").  Targets: real points of a leaf (kind 0) or the UC (1) /
-// DC (2) check surface of a node.  Entries: (kind << 28) | node, kind 0 =
-// the node's source points, 1 = the node's UE surface carrying uden, 2 = the
-// node's DE surface carrying dden.  Output: out[job.out + i] = (or +=)
+// DC (2) check surface of a node.  Entries: `count` sources, kind 0 = source
+// points from leaf-order position `base` on (of leaf `node`; plain plans merge
+// adjacent leaves' ranges), 1 = node's UE surface carrying uden, 2 = the node's
+// DE surface carrying dden (base 0).  Output: out[job.out + i] = (or +=)
 // 1/(4 pi) sum_j w_j / |t_i - s_j|, pairs with r == 0 skipped
 // (fmm/omp.cc:259-283).
 // ---------------------------------------------------------------------------
+struct __align__(16) P2PEntry {
+  int base, count, kind, node;
+};
+
 struct P2PJob {
   int tnode, tkind, tbeg, tcnt;
   int ebeg, eend, out, mode;  // mode 0 write, 1 add
+  int ns;    // sources of all entries
+  int plan;  // batched solves: whose arrays
+  int copies;  // team jobs of at most 16 or 8 targets: 2 or 4 copies of them in a warp
 };
 
 struct P2PParams {
   const P2PJob* jobs;
-  const int* entries;
+  const P2PEntry* entries;
   const double4* src4;
   const double4* trg4;
   const double4* ctr;
-  const int* src_beg;
-  const int* src_num;
   const double* uden;
   const double* dden;
   const double* sp_ue;  // 3 per point
@@ -67,6 +73,12 @@ struct P2PMixedParams {
   const float4* ctrf;
   const float* spf_ue;  // the unit UE / DE surfaces in FP32, 3 per point
   const float* spf_de;
+  // the entries as (kind << 28) | node for the row jobs' cursor, which reads the
+  // leaf ranges itself (one 16-byte entry load instead costs registers there:
+  // S2M of 4M points, NP 6, 0.397 -> 0.415 ms)
+  const int* entry_ids;
+  const int* src_beg;
+  const int* src_num;
   // near field: target i of a job goes to out[out_perm[J.out + i]], the
   // original order (no scatter pass afterwards); null: out[J.out + i]
   const int* out_perm;
@@ -118,18 +130,6 @@ constexpr int kMaxSlots = 6;  // targets per lane: jobs hold up to 192 targets
 #define KFMM_P2P_MIXED_MINB 6  // resident blocks per SM asked of the mixed P2P kernel
 #endif
 
-__device__ __forceinline__ void load_entry_source(const P2PParams& p, int kind, int node,
-                                                  int base, int idx, double3& s, double& w) {
-  if (kind == 0) {
-    const double4 v = p.src4[base + idx];
-    s = make_double3(v.x, v.y, v.z);
-    w = v.w;
-  } else {
-    s = surface_point(p.ctr[node], kind == 1 ? p.sp_ue : p.sp_de, idx);
-    w = (kind == 1 ? p.uden : p.dden)[(size_t)node * p.P + idx];
-  }
-}
-
 // 1 / sqrt(r2) in FP64 for the pair sums.  The seed is the approximate reciprocal
 // square root (PTX rsqrt.approx.ftz.f64, one MUFU operation), followed by one
 // third-order Householder step for y^-2 = r2 (A. S. Householder, The Numerical
@@ -158,14 +158,15 @@ __device__ __forceinline__ double pair_rsqrt(double r2) {
   return y;
 }
 
-template <int NS, bool kGuard>
+// `cnt` sources at every G-th place of buf.
+template <int NS, bool kGuard, int G = 1>
 __device__ __forceinline__ void pairs_fp64(const double (&tx)[NS], const double (&ty)[NS],
                                            const double (&tz)[NS], double (&acc)[NS],
                                            const double4* buf, int cnt) {
   constexpr int kUnroll = NS >= 4 ? 2 : NS >= 2 ? 4 : 8;  // chains in flight: 8 to 12
 #pragma unroll kUnroll
   for (int k = 0; k < cnt; ++k) {
-    const double4 s = buf[k];
+    const double4 s = buf[k * G];
 #pragma unroll
     for (int t = 0; t < NS; ++t) {
       const double dx = tx[t] - s.x, dy = ty[t] - s.y, dz = tz[t] - s.z;
@@ -285,7 +286,7 @@ __device__ __forceinline__ float pair_term1(float tx, float ty, float tz, float 
 // conversions take XU slots beside the reciprocal square roots: blocks of 16
 // measured 0.11 ms slower at 4M points, with a 2% smaller rel-L2 error.)
 // buf: per source {x,x},{y,y} then {z,z},{w,w} (two ulonglong2 per source).
-template <int NS, bool kGuard>
+template <int NS, bool kGuard, int G = 1>
 __device__ __forceinline__ void pairs_mixed(const unsigned long long (&tx)[(NS + 1) / 2],
                                             const unsigned long long (&ty)[(NS + 1) / 2],
                                             const unsigned long long (&tz)[(NS + 1) / 2],
@@ -298,17 +299,20 @@ __device__ __forceinline__ void pairs_mixed(const unsigned long long (&tx)[(NS +
 #pragma unroll
     for (int t = 0; t < NP2; ++t) blk[t] = 0ull;
     auto step = [&](int u) {
-      const ulonglong2 a = buf[2 * (k + u)], b = buf[2 * (k + u) + 1];
+      const ulonglong2 a = buf[2 * G * (k + u)], b = buf[2 * G * (k + u) + 1];
 #pragma unroll
       for (int t = 0; t < NP2; ++t) blk[t] = pair_term2<kGuard>(tx[t], ty[t], tz[t], a, b, blk[t]);
       if (ODD)
         blk1 = pair_term1<kGuard>(lo_of(tx[NP2]), lo_of(ty[NP2]), lo_of(tz[NP2]), lo_of(a.x),
                                   lo_of(a.y), lo_of(b.x), lo_of(b.y), blk1);
     };
-    if (m == kBlock) {
+    if (G == 1 && m == kBlock) {
       constexpr int kUnroll = NS > 4 ? 2 : 4;  // bounds the live pair temporaries
 #pragma unroll kUnroll
       for (int u = 0; u < kBlock; ++u) step(u);
+    } else if (G > 1) {
+#pragma unroll 4
+      for (int u = 0; u < m; ++u) step(u);
     } else {
       for (int u = 0; u < m; ++u) step(u);
     }
@@ -340,13 +344,12 @@ struct EntryCursor {
   float3 dlt;
   float rad;
   __device__ __forceinline__ void open(const P2PMixedParams& a, const float4 orgf) {
-    const P2PParams& p = a.p;
     for (; e < eend; ++e) {
-      const int ent = p.entries[e];
+      const int ent = a.entry_ids[e];
       kind = ent >> 28;
       node = ent & 0x0fffffff;
-      count = kind == 0 ? p.src_num[node] : p.P;
-      base = kind == 0 ? p.src_beg[node] : 0;
+      count = kind == 0 ? a.src_num[node] : a.p.P;
+      base = kind == 0 ? a.src_beg[node] : 0;
       if (count > 0) break;
     }
     if (e < eend) {
@@ -380,8 +383,8 @@ struct EntryCursor {
 // is target l + 32k; each chunk of 32 sources goes through the warp's shared
 // buffer in the target node's FP32 frame and is read back as broadcasts.
 template <int NS>
-__device__ __forceinline__ void warp_job_mixed(const P2PMixedParams& a, const P2PJob& J, int lane,
-                                               void* wbuf) {
+__device__ __forceinline__ void row_job_mixed(const P2PMixedParams& a, const P2PJob& J, int lane,
+                                              void* wbuf) {
   const P2PParams& p = a.p;
   const double4 org = p.ctr[J.tnode];
   const float4 orgf = a.ctrf[J.tnode];
@@ -441,112 +444,312 @@ __device__ __forceinline__ void warp_job_mixed(const P2PMixedParams& a, const P2
   }
 }
 
-// Plain FP64 form of a row job: the same walk, sources staged as double4.
-template <int NS>
-__device__ __forceinline__ void warp_job_fp64(const P2PParams& p, const P2PJob& J, int lane,
-                                              void* wbuf) {
-  const double4 org = p.ctr[J.tnode];
-  double q[NS][3];
+// A warp's walk over its share [lo, hi) of a job's sources, 32 at a time.  The
+// job's entries are read 32 at once, one per lane, cut to the share and staged in
+// the warp's shared memory (the mixed form with each entry node's centre relative
+// to the target node's, exact in FP32, and its radius), so that going from one
+// entry to the next costs one shared load and no dependent global loads.
+template <bool kMixed>
+struct __align__(16) EntryStage {
+  P2PEntry ent[32];
+  float4 off[kMixed ? 32 : 1];
+};
+
+template <bool kMixed>
+struct Walk {
+  int e, eend, lo, hi;  // next entry to stage; the share, relative to its first source
+  int i, m, c0;         // entry i of the m staged ones, its sources from c0 on
+  P2PEntry q;           // entry i
+  __device__ __forceinline__ bool refill(const P2PArgs<kMixed>& a, const float4 orgf, int lane,
+                                         EntryStage<kMixed>* st) {
+    while (e < eend && hi > 0) {
+      P2PEntry t{0, 0, 0, 0};
+      if (e + lane < eend) t = base_of(a).entries[e + lane];
+      int end = t.count;
 #pragma unroll
-  for (int t = 0; t < NS; ++t) {
-    const int i = lane + 32 * t;
-    double3 v = make_double3(org.x, org.y, org.z);
-    if (i < J.tcnt) {
-      if (J.tkind == 0) {
-        const double4 w = p.trg4[J.tbeg + i];
-        v = make_double3(w.x, w.y, w.z);
-      } else {
-        v = surface_point(org, J.tkind == 1 ? p.sp_uc : p.sp_dc, J.tbeg + i);
+      for (int d = 1; d < 32; d *= 2) {
+        const int v = __shfl_up_sync(0xffffffffu, end, d);
+        if (lane >= d) end += v;
+      }
+      const int start = end - t.count, from = max(start, lo), n = min(end, hi) - from;
+      const unsigned keep = __ballot_sync(0xffffffffu, n > 0);
+      const int all = __shfl_sync(0xffffffffu, end, 31);
+      e += 32;
+      lo -= all;
+      hi -= all;
+      if (keep) {
+        __syncwarp();
+        if (n > 0) {
+          const int slot = __popc(keep & ((1u << lane) - 1u));
+          st->ent[slot] = P2PEntry{t.base + from - start, n, t.kind, t.node};
+          if constexpr (kMixed) {
+            const float4 k = a.ctrf[t.node];
+            st->off[slot] = make_float4(k.x - orgf.x, k.y - orgf.y, k.z - orgf.z, k.w);
+          }
+        }
+        __syncwarp();
+        i = 0;
+        m = __popc(keep);
+        c0 = 0;
+        q = st->ent[0];
+        return true;
       }
     }
-    q[t][0] = v.x;
-    q[t][1] = v.y;
-    q[t][2] = v.z;
+    return false;
   }
-  // chunk cursor over the job's entries: entry e, sources [c0, c0 + 32)
-  int e = J.ebeg, c0 = 0, kind = 0, node = 0, count = 0, base = 0;
-  auto open_entry = [&]() {  // first entry at or after e with sources
-    for (; e < J.eend; ++e) {
-      const int ent = p.entries[e];
-      kind = ent >> 28;
-      node = ent & 0x0fffffff;
-      count = kind == 0 ? p.src_num[node] : p.P;
-      base = kind == 0 ? p.src_beg[node] : 0;
-      if (count > 0) return;
+  // the next 32 sources; false at the end
+  __device__ __forceinline__ bool advance(const P2PArgs<kMixed>& a, const float4 orgf, int lane,
+                                          EntryStage<kMixed>* st) {
+    c0 += 32;
+    if (c0 < q.count) return true;
+    if (++i < m) {
+      c0 = 0;
+      q = st->ent[i];
+      return true;
     }
-  };
-  open_entry();
-  double3 s = make_double3(0.0, 0.0, 0.0);
-  double w = 0.0;
-  if (e < J.eend && lane < min(32, count - c0)) load_entry_source(p, kind, node, base, c0 + lane, s, w);
+    return refill(a, orgf, lane, st);
+  }
+};
 
-  double sum[NS];
-  {
-    double tx[NS], ty[NS], tz[NS], acc[NS];
+// Source c0 + lane of the walk's entry.  Plain form: absolute coordinates.
+__device__ __forceinline__ double4 walk_source(const P2PParams& p, const Walk<false>& w, int lane) {
+  const int idx = w.q.base + w.c0 + lane;
+  if (w.q.kind == 0) return p.src4[idx];
+  const double3 s = surface_point(p.ctr[w.q.node], w.q.kind == 1 ? p.sp_ue : p.sp_de, idx);
+  return make_double4(s.x, s.y, s.z,
+                      (w.q.kind == 1 ? p.uden : p.dden)[(size_t)w.q.node * p.P + idx]);
+}
+// Mixed form: relative to the entry node's centre (the leaf point's stored
+// offset, or radius * FP32 unit-surface point, which is exact); the entry's
+// offset is added when the chunk is written to the warp's buffer, so this load
+// stays in flight across the pair loop.
+__device__ __forceinline__ float4 walk_source(const P2PMixedParams& a, const Walk<true>& w,
+                                              int lane, const EntryStage<true>* st) {
+  const int idx = w.q.base + w.c0 + lane;
+  if (w.q.kind == 0) return a.src4f[idx];
+  const float* sp = (w.q.kind == 1 ? a.spf_ue : a.spf_de) + 3 * idx;
+  const double v = (w.q.kind == 1 ? a.p.uden : a.p.dden)[(size_t)w.q.node * a.p.P + idx];
+  const float rad = st->off[w.i].w;
+  return make_float4(rad * sp[0], rad * sp[1], rad * sp[2], (float)v);
+}
+
+// The warps of a team (one CTA) share a job's sources; their sums meet in `red`
+// and are added in warp order.
+constexpr int kTeam = kWarpJobsPerBlock;
+constexpr int kTeamRows = 4;  // targets per lane: a team's jobs hold up to 128
+struct TeamSums {
+  double v[kTeam][32 * kTeamRows];
+};
+
+__device__ __forceinline__ void store_sum(const P2PJob& J, double* out, const int* perm, int i,
+                                          double sum) {
+  double* o = out + (perm ? perm[J.out + i] : J.out + i);
+  const double r = kOOFP * sum;
+  if (J.mode) *o += r;
+  else *o = r;
+}
+
+template <int NS, int G, bool kIsTeam>
+__device__ __forceinline__ void store_job(const P2PJob& J, double* out, const int* perm,
+                                          double (&acc)[NS], int lane, TeamSums* red) {
+#pragma unroll
+  for (int d = 32 / G; d < 32; d *= 2) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], d);
+  if constexpr (!kIsTeam) {
 #pragma unroll
     for (int t = 0; t < NS; ++t) {
-      tx[t] = q[t][0];
-      ty[t] = q[t][1];
-      tz[t] = q[t][2];
-      acc[t] = 0.0;
+      const int i = lane + 32 * t;
+      if (i < J.tcnt) store_sum(J, out, perm, i, acc[t]);
     }
-    double4* buf = (double4*)wbuf;
-    while (e < J.eend) {
-      const int cnt = min(32, count - c0);
-      const bool guard = kind == 0 && J.tkind == 0 && node == J.tnode;
-      if (lane < cnt) buf[lane] = make_double4(s.x, s.y, s.z, w);
-      __syncwarp();
-      c0 += 32;
-      if (c0 >= count) {
-        ++e;
-        c0 = 0;
-        open_entry();
-      }
-      if (e < J.eend && lane < min(32, count - c0))
-        load_entry_source(p, kind, node, base, c0 + lane, s, w);
-      if (guard) pairs_fp64<NS, true>(tx, ty, tz, acc, buf, cnt);
-      else pairs_fp64<NS, false>(tx, ty, tz, acc, buf, cnt);
-      __syncwarp();
-    }
+  } else {
+    const int wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int t = 0; t < NS; ++t) sum[t] = acc[t];
-  }
+    for (int t = 0; t < NS; ++t) red->v[wid][lane + 32 * t] = acc[t];
+    __syncthreads();
+    for (int i = threadIdx.x; i < J.tcnt; i += 32 * kTeam) {
+      double s = red->v[0][i];
 #pragma unroll
-  for (int t = 0; t < NS; ++t) {
-    const int i = lane + 32 * t;
-    if (i < J.tcnt) {
-      const double r = kOOFP * sum[t];
-      double* o = p.out + J.out + i;
-      if (J.mode) *o += r;
-      else *o = r;
+      for (int w = 1; w < kTeam; ++w) s += red->v[w][i];
+      store_sum(J, out, perm, i, s);
     }
   }
 }
 
+// A warp's part of a job: slot k of lane l is target l + 32k (G = 1).  Jobs of G =
+// 2 or 4 copies hold at most 32 / G targets, copy g meeting every G-th source (one
+// slot; chunks are then padded with sources of zero weight).
+template <bool kIsTeam, bool kMixed>
+__device__ __forceinline__ Walk<kMixed> walk_of(const P2PJob& J) {
+  Walk<kMixed> w{};
+  w.e = J.ebeg;
+  w.eend = J.eend;
+  w.hi = J.ns;
+  if constexpr (kIsTeam) {
+    const int wid = threadIdx.x >> 5, chunks = (J.ns + 31) >> 5;
+    w.lo = 32 * ((chunks * wid) / kTeam);
+    w.hi = min(J.ns, 32 * ((chunks * (wid + 1)) / kTeam));
+  }
+  return w;
+}
+
+template <int NS, int G>
+__device__ __forceinline__ void team_job_mixed(const P2PMixedParams& a, const P2PJob& J, int lane,
+                                               void* wbuf, EntryStage<true>* st, TeamSums* red) {
+  const P2PParams& p = a.p;
+  const double4 org = p.ctr[J.tnode];
+  const float4 orgf = a.ctrf[J.tnode];
+  constexpr int NP2C = (NS + 1) / 2;
+  unsigned long long tx[NP2C], ty[NP2C], tz[NP2C];
+  {
+    float q[NS][3];
+#pragma unroll
+    for (int t = 0; t < NS; ++t) {
+      const int i = G > 1 ? lane % (32 / G) : lane + 32 * t;
+      double3 v = make_double3(org.x, org.y, org.z);
+      if (i < J.tcnt) v = job_target(p, J, org, i);
+      q[t][0] = (float)(v.x - org.x);
+      q[t][1] = (float)(v.y - org.y);
+      q[t][2] = (float)(v.z - org.z);
+    }
+#pragma unroll
+    for (int t = 0; t < NP2C; ++t) {
+      const int u = 2 * t + 1 < NS ? 2 * t + 1 : 2 * t;
+      tx[t] = pack2(q[2 * t][0], q[u][0]);
+      ty[t] = pack2(q[2 * t][1], q[u][1]);
+      tz[t] = pack2(q[2 * t][2], q[u][2]);
+    }
+  }
+  Walk<true> w = walk_of<true, true>(J);
+  bool more = w.refill(a, orgf, lane, st);
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (more && lane < w.q.count) s = walk_source(a, w, lane, st);
+  double acc[NS];
+#pragma unroll
+  for (int t = 0; t < NS; ++t) acc[t] = 0.0;
+  ulonglong2* buf = (ulonglong2*)wbuf;
+  while (more) {
+    int cnt = min(32, w.q.count - w.c0);
+    const bool guard = w.q.kind == 0 && J.tkind == 0 && w.q.node == J.tnode;
+    if (lane < cnt) {
+      const float4 o = st->off[w.i];
+      const float x = s.x + o.x, y = s.y + o.y, z = s.z + o.z;
+      buf[2 * lane] = make_ulonglong2(pack2(x, x), pack2(y, y));
+      buf[2 * lane + 1] = make_ulonglong2(pack2(z, z), pack2(s.w, s.w));
+    } else if (G > 1) {
+      // outside every target's box, weight zero
+      buf[2 * lane] = make_ulonglong2(pack2(8.f, 8.f), pack2(8.f, 8.f));
+      buf[2 * lane + 1] = make_ulonglong2(pack2(8.f, 8.f), 0ull);
+    }
+    __syncwarp();
+    more = w.advance(a, orgf, lane, st);
+    if (more && lane < w.q.count - w.c0) s = walk_source(a, w, lane, st);
+    if constexpr (G > 1) {
+      cnt = (cnt + G - 1) / G;
+      const ulonglong2* mine = buf + 2 * (lane / (32 / G));
+      if (guard) pairs_mixed<NS, true, G>(tx, ty, tz, acc, mine, cnt);
+      else pairs_mixed<NS, false, G>(tx, ty, tz, acc, mine, cnt);
+    } else {
+      if (guard) pairs_mixed<NS, true>(tx, ty, tz, acc, buf, cnt);
+      else pairs_mixed<NS, false>(tx, ty, tz, acc, buf, cnt);
+    }
+    __syncwarp();
+  }
+  store_job<NS, G, true>(J, p.out, a.out_perm, acc, lane, red);
+}
+
+// Plain FP64 form: the same walk, sources staged as double4.
+template <int NS, int G, bool kIsTeam>
+__device__ __forceinline__ void warp_job_fp64(const P2PParams& p, const P2PJob& J, int lane,
+                                              void* wbuf, EntryStage<false>* st, TeamSums* red) {
+  const double4 org = p.ctr[J.tnode];
+  double tx[NS], ty[NS], tz[NS], acc[NS];
+#pragma unroll
+  for (int t = 0; t < NS; ++t) {
+    const int i = G > 1 ? lane % (32 / G) : lane + 32 * t;
+    double3 v = make_double3(org.x, org.y, org.z);
+    if (i < J.tcnt) v = job_target(p, J, org, i);
+    tx[t] = v.x;
+    ty[t] = v.y;
+    tz[t] = v.z;
+    acc[t] = 0.0;
+  }
+  Walk<false> w = walk_of<kIsTeam, false>(J);
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+  bool more = w.refill(p, none, lane, st);
+  double4 s = make_double4(0.0, 0.0, 0.0, 0.0);
+  if (more && lane < w.q.count) s = walk_source(p, w, lane);
+  double4* buf = (double4*)wbuf;
+  while (more) {
+    const int cnt = min(32, w.q.count - w.c0);
+    const bool guard = w.q.kind == 0 && J.tkind == 0 && w.q.node == J.tnode;
+    if (lane < cnt) buf[lane] = s;
+    else if (G > 1) buf[lane] = make_double4(0.0, 0.0, 0.0, 0.0);
+    __syncwarp();
+    more = w.advance(p, none, lane, st);
+    if (more && lane < w.q.count - w.c0) s = walk_source(p, w, lane);
+    const double4* mine = G > 1 ? buf + lane / (32 / G) : buf;
+    if (guard) pairs_fp64<NS, true, G>(tx, ty, tz, acc, mine, (cnt + G - 1) / G);
+    else pairs_fp64<NS, false, G>(tx, ty, tz, acc, mine, (cnt + G - 1) / G);
+    __syncwarp();
+  }
+  store_job<NS, G, kIsTeam>(J, p.out, nullptr, acc, lane, red);
+}
+
+// Shared memory of one P2P warp: its chunk of 32 sources and its staged entries.
+template <bool kMixed>
+struct __align__(16) P2PWarpSmem {
+  unsigned char chunk[32 * 32];
+  EntryStage<kMixed> st;
+};
+
+// One warp per job: the mixed form walks with its cursor (row_job_mixed), the plain
+// form as a team of one.
+template <bool kMixed>
+using P2PRowSmem = typename std::conditional<kMixed, unsigned char[32 * 32], P2PWarpSmem<false>>::type;
+
 template <bool kMixed, int NS>
 __device__ __forceinline__ void warp_job(const P2PArgs<kMixed>& a, const P2PJob& J, int lane,
-                                         void* wbuf) {
-  if constexpr (kMixed) warp_job_mixed<NS>(a, J, lane, wbuf);
-  else warp_job_fp64<NS>(a, J, lane, wbuf);
+                                         void* ws) {
+  if constexpr (kMixed) {
+    row_job_mixed<NS>(a, J, lane, ws);
+  } else {
+    P2PWarpSmem<false>* w = (P2PWarpSmem<false>*)ws;
+    warp_job_fp64<NS, 1, false>(a, J, lane, w->chunk, &w->st, nullptr);
+  }
 }
 
 template <bool kMixed>
 __device__ __forceinline__ void run_job(const P2PArgs<kMixed>& a, const P2PJob& J, int lane,
-                                        void* wb) {
+                                        void* ws) {
   switch ((J.tcnt + 31) >> 5) {
-    case 1: warp_job<kMixed, 1>(a, J, lane, wb); break;
-    case 2: warp_job<kMixed, 2>(a, J, lane, wb); break;
-    case 3: warp_job<kMixed, 3>(a, J, lane, wb); break;
-    case 4: warp_job<kMixed, 4>(a, J, lane, wb); break;
-    case 5: warp_job<kMixed, 5>(a, J, lane, wb); break;
-    default: warp_job<kMixed, kMaxSlots>(a, J, lane, wb); break;
+    case 1: warp_job<kMixed, 1>(a, J, lane, ws); break;
+    case 2: warp_job<kMixed, 2>(a, J, lane, ws); break;
+    case 3: warp_job<kMixed, 3>(a, J, lane, ws); break;
+    case 4: warp_job<kMixed, 4>(a, J, lane, ws); break;
+    case 5: warp_job<kMixed, 5>(a, J, lane, ws); break;
+    default: warp_job<kMixed, kMaxSlots>(a, J, lane, ws); break;
   }
 }
 
-__device__ __forceinline__ int next_job_of_warp(int* next_job, int lane) {
-  int j = 0;
-  if (lane == 0) j = atomicAdd(next_job, 1);
-  return __shfl_sync(0xffffffffu, j, 0);
+template <bool kMixed, int NS, int G>
+__device__ __forceinline__ void team_job(const P2PArgs<kMixed>& a, const P2PJob& J, int lane,
+                                         P2PWarpSmem<kMixed>* ws, TeamSums* red) {
+  if constexpr (kMixed) team_job_mixed<NS, G>(a, J, lane, ws->chunk, &ws->st, red);
+  else warp_job_fp64<NS, G, true>(a, J, lane, ws->chunk, &ws->st, red);
+}
+
+template <bool kMixed>
+__device__ __forceinline__ void run_team_job(const P2PArgs<kMixed>& a, const P2PJob& J, int lane,
+                                             P2PWarpSmem<kMixed>* ws, TeamSums* red) {
+  switch ((J.tcnt + 31) >> 5) {
+    case 1:
+      if (J.copies == 4) team_job<kMixed, 1, 4>(a, J, lane, ws, red);
+      else if (J.copies == 2) team_job<kMixed, 1, 2>(a, J, lane, ws, red);
+      else team_job<kMixed, 1, 1>(a, J, lane, ws, red);
+      break;
+    case 2: team_job<kMixed, 2, 1>(a, J, lane, ws, red); break;
+    case 3: team_job<kMixed, 3, 1>(a, J, lane, ws, red); break;
+    default: team_job<kMixed, kTeamRows, 1>(a, J, lane, ws, red); break;
+  }
 }
 
 // Persistent: each warp takes jobs from *next_job until none are left.  The
@@ -558,35 +761,59 @@ __device__ __forceinline__ int next_job_of_warp(int* next_job, int lane) {
 template <bool kMixed, int kMinBlocks = kMixed ? KFMM_P2P_MIXED_MINB : 4>
 __global__ void __launch_bounds__(32 * kWarpJobsPerBlock, kMinBlocks)
 p2p_warp_kernel(P2PArgs<kMixed> a, int njobs, int* next_job) {
-  __shared__ __align__(16) unsigned char smem[kWarpJobsPerBlock][32 * 32];
+  __shared__ __align__(16) P2PRowSmem<kMixed> smem[kWarpJobsPerBlock];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  void* wb = smem[wid];
   for (;;) {
     int j = 0;
     if (lane == 0) j = atomicAdd(next_job, 1);
     j = __shfl_sync(0xffffffffu, j, 0);
     if (j >= njobs) return;
     const P2PJob J = base_of(a).jobs[j];  // a register copy: the output stores may alias
-    run_job<kMixed>(a, J, lane, wb);
+    run_job<kMixed>(a, J, lane, &smem[wid]);
   }
 }
 
-// The near fields of many plans in one persistent launch (batched solves):
-// job j is job jobs[j].y of plan jobs[j].x, whose arrays params[jobs[j].x]
-// describes.
+// One job per CTA, its sources shared by the CTA's four warps; blocks start in
+// job order, largest first.  A job's time is a quarter of what one warp takes, so
+// near fields with few jobs per resident warp neither wait for the longest of
+// them nor leave warps idle: 65,536 points NP 4 plain 0.95 -> 0.16 ms, 1M points
+// NP 6 mixed 2.17 -> 1.92 ms.  Resident blocks asked of ptxas: plain 4 (119
+// registers; 5 and 6 measured 2% slower at 4M points), mixed 8 (64 registers; 5 to
+// 7 measured 1-5% slower at 1M and 4M).
+constexpr int kTeamBlocksFp64 = 4, kTeamBlocksMixed = 8;
+
 template <bool kMixed>
-__global__ void __launch_bounds__(32 * kWarpJobsPerBlock, kMixed ? KFMM_P2P_MIXED_MINB : 4)
-p2p_fused_kernel(const P2PArgs<kMixed>* params, const int2* jobs, int njobs, int* next_job) {
+__global__ void __launch_bounds__(32 * kTeam, kMixed ? kTeamBlocksMixed : kTeamBlocksFp64)
+p2p_team_kernel(P2PArgs<kMixed> a) {
+  __shared__ P2PWarpSmem<kMixed> smem[kTeam];
+  __shared__ TeamSums red;
+  const P2PJob J = base_of(a).jobs[blockIdx.x];
+  run_team_job<kMixed>(a, J, threadIdx.x & 31, &smem[threadIdx.x >> 5], &red);
+}
+
+// The near fields of many plans in one launch (batched solves): job j is of the
+// plan whose arrays params[jobs[j].plan] describes.
+template <bool kMixed>
+__global__ void __launch_bounds__(32 * kTeam, kMixed ? kTeamBlocksMixed : kTeamBlocksFp64)
+p2p_team_batch_kernel(const P2PArgs<kMixed>* params, const P2PJob* jobs) {
+  __shared__ P2PWarpSmem<kMixed> smem[kTeam];
+  __shared__ TeamSums red;
+  const P2PJob J = jobs[blockIdx.x];
+  run_team_job<kMixed>(params[J.plan], J, threadIdx.x & 31, &smem[threadIdx.x >> 5], &red);
+}
+
+// The same with one warp per job (mixed plans with jobs enough).
+__global__ void __launch_bounds__(32 * kWarpJobsPerBlock, KFMM_P2P_MIXED_MINB)
+p2p_fused_kernel(const P2PMixedParams* params, const P2PJob* jobs, int njobs, int* next_job) {
   __shared__ __align__(16) unsigned char smem[kWarpJobsPerBlock][32 * 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  void* wb = smem[wid];
   for (;;) {
-    const int j = next_job_of_warp(next_job, lane);
+    int j = 0;
+    if (lane == 0) j = atomicAdd(next_job, 1);
+    j = __shfl_sync(0xffffffffu, j, 0);
     if (j >= njobs) return;
-    const int2 pj = jobs[j];
-    const P2PArgs<kMixed>& a = params[pj.x];
-    const P2PJob J = base_of(a).jobs[pj.y];
-    run_job<kMixed>(a, J, lane, wb);
+    const P2PJob J = jobs[j];
+    run_job<true>(params[J.plan], J, lane, smem[wid]);
   }
 }
 

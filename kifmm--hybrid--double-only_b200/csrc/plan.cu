@@ -74,7 +74,8 @@ struct kfmm_plan {
   std::vector<void*> allocs;
   // tree on device
   double4* ctr = nullptr;
-  int *d_depth = nullptr, *d_src_beg = nullptr, *d_src_num = nullptr;
+  int* d_depth = nullptr;
+  int *d_src_beg = nullptr, *d_src_num = nullptr;  // mixed form: leaf ranges for the cursors
   int *d_src_perm = nullptr, *d_trg_perm = nullptr;
   int *d_src_inv = nullptr, *d_trg_inv = nullptr;  // original index -> leaf-order position
   // points
@@ -102,14 +103,15 @@ struct kfmm_plan {
   int *d_surf_idx = nullptr, *d_surf_ijk = nullptr;
   // work lists
   P2PJob *s2m_jobs = nullptr, *nf_jobs = nullptr, *s2l_jobs = nullptr;
-  int *s2m_ent = nullptr, *nf_ent = nullptr, *s2l_ent = nullptr;
+  // their entries; the row jobs of mixed plans take them as (kind << 28) | node
+  P2PEntry *s2m_ent = nullptr, *nf_ent = nullptr, *s2l_ent = nullptr;
+  int *s2m_ids = nullptr, *nf_ids = nullptr, *s2l_ids = nullptr;
   int n_s2m = 0, n_nf = 0, n_s2l = 0;
-  std::vector<float> nf_class;  // cost class of each near-field job (-log1.25 cost)
   // the near field's jobs before chunking (one per target leaf, all its
-  // targets) and their source counts, kept to re-chunk on a new job size
+  // targets), kept to re-chunk on a new job size
   std::vector<P2PJob> nf_leaf;
-  std::vector<double> nf_leaf_ns;
   bool nf_w_heavy = false;     // W-list surfaces carry > 1% of the near-field pairs
+  bool nf_team = false;        // near field in team jobs (p2p_team_kernel)
   int* job_counter = nullptr;  // persistent P2P work counters: S2M, S2L, near field
   // [0] set by kernels whose bounded waits ran out, zeroed per solve; [1]
   // collects [0] over the kfmm_evaluate_async calls since the last wait
@@ -330,15 +332,13 @@ kfmm_status launch_gemms(const kfmm_plan* p, const std::vector<GemmBatch>& gs, c
   return KFMM_OK;
 }
 
-P2PParams p2p_params(const kfmm_plan* p, const P2PJob* jobs, const int* ent, double* out) {
+P2PParams p2p_params(const kfmm_plan* p, const P2PJob* jobs, const P2PEntry* ent, double* out) {
   P2PParams q;
   q.jobs = jobs;
   q.entries = ent;
   q.src4 = p->src4;
   q.trg4 = p->trg4;
   q.ctr = p->ctr;
-  q.src_beg = p->d_src_beg;
-  q.src_num = p->d_src_num;
   q.uden = p->uden;
   q.dden = p->dden;
   q.sp_ue = p->d_sp_ue;
@@ -351,7 +351,7 @@ P2PParams p2p_params(const kfmm_plan* p, const P2PJob* jobs, const int* ent, dou
   return q;
 }
 
-P2PMixedParams p2p_mixed_params(const kfmm_plan* p, const P2PParams& q,
+P2PMixedParams p2p_mixed_params(const kfmm_plan* p, const P2PParams& q, const int* ids,
                                 const int* out_perm = nullptr) {
   P2PMixedParams m;
   m.p = q;
@@ -360,6 +360,9 @@ P2PMixedParams p2p_mixed_params(const kfmm_plan* p, const P2PParams& q,
   m.spf_ue = p->d_spf_ue;
   m.spf_de = p->d_spf_de;
   m.out_perm = out_perm;
+  m.entry_ids = ids;
+  m.src_beg = p->d_src_beg;
+  m.src_num = p->d_src_num;
   return m;
 }
 
@@ -455,39 +458,16 @@ inline long long key_of(int x, int y, int z) {
 
 constexpr double kCostClassWidth = 1.05;  // cost ratio spanned by one job-order class
 
-// The near field's jobs: each target leaf's targets in chunks of 32 * rows
-// (rows: the tuning's job_rows, else 4 for mixed plans whose W-list surfaces
-// carry more than 1% of the pairs, else 6), ordered largest first by cost
-// class (target slots x sources, in classes 5% wide); within a class the
-// jobs keep their tree order, so warps working at the same time read
-// neighbouring leaves' sources and the L2 cache serves the repeats (4M
-// points, NP=6 uniform / NP=4 ellipsoid surface, mixed near field: classes
-// 25% wide 4.44 / 2.32 ms, 12% 4.39 / 2.28, 5% 4.39 / 2.27, 100% 4.48 /
-// 2.50).  The
-// mixed near field runs with 5 resident blocks per SM on the same clouds
-// (or when the tuning says so).  Measured on 4M points on the ellipsoid
-// surface, NP=4, 256 per box: 2.32 ms against 2.50 ms with 6 blocks and 6
-// rows; uniform clouds keep 6 and 6 (4.42 ms, against 4.70 ms with 4 rows).
-kfmm_status build_nf_jobs(kfmm_plan* p) {
-  int rows = p->prec == KFMM_MIXED && p->nf_w_heavy ? 4 : kMaxSlots;
-  if (p->tune.job_rows > 0) rows = std::min(p->tune.job_rows, kMaxSlots);
-  const int chunk = 32 * rows;
-  std::vector<P2PJob> jobs;
-  std::vector<double> ns;
-  for (size_t l = 0; l < p->nf_leaf.size(); ++l) {
-    const P2PJob& L = p->nf_leaf[l];
-    for (int c = 0; c < L.tcnt; c += chunk) {
-      P2PJob j = L;
-      j.tbeg = L.tbeg + c;
-      j.tcnt = std::min(chunk, L.tcnt - c);
-      j.out = L.out + c;
-      jobs.push_back(j);
-      ns.push_back(p->nf_leaf_ns[l]);
-    }
-  }
+// Order of P2P jobs: largest first by cost class (target slots x sources, in
+// classes 5% wide); within a class the jobs keep their tree order, so warps
+// working at the same time read neighbouring leaves' sources and the L2 cache
+// serves the repeats (4M points, NP=6 uniform / NP=4 ellipsoid surface, mixed near
+// field: classes 25% wide 4.44 / 2.32 ms, 12% 4.39 / 2.28, 5% 4.39 / 2.27, 100%
+// 4.48 / 2.50).
+void order_jobs(std::vector<P2PJob>& jobs) {
   std::vector<std::pair<double, int>> key(jobs.size());
   for (size_t j = 0; j < jobs.size(); ++j) {
-    const double cost = std::max(1.0, ns[j] * ((jobs[j].tcnt + 31) / 32));
+    const double cost = std::max(1.0, (double)jobs[j].ns * ((jobs[j].tcnt + 31) / 32));
     key[j] = {-std::floor(std::log(cost) / std::log(kCostClassWidth)), (int)j};
   }
   std::stable_sort(key.begin(), key.end(),
@@ -495,14 +475,91 @@ kfmm_status build_nf_jobs(kfmm_plan* p) {
                      return a.first < b.first;
                    });
   std::vector<P2PJob> out(jobs.size());
-  p->nf_class.resize(jobs.size());
-  for (size_t j = 0; j < jobs.size(); ++j) {
-    out[j] = jobs[key[j].second];
-    p->nf_class[j] = (float)key[j].first;
+  for (size_t j = 0; j < jobs.size(); ++j) out[j] = jobs[key[j].second];
+  jobs.swap(out);
+}
+
+// Appends the targets [from, to) of a job over all its targets.
+void add_part(std::vector<P2PJob>& jobs, const P2PJob& all, int from, int to) {
+  P2PJob j = all;
+  j.tbeg += from;
+  j.tcnt = to - from;
+  j.out += from;
+  jobs.push_back(j);
+}
+
+// A job's targets in parts of nearly equal numbers of 32-target rows, at most
+// `rows` each.
+void split_even(std::vector<P2PJob>& jobs, const P2PJob& all, int count, int rows) {
+  const int full = (count + 31) / 32, parts = (full + rows - 1) / rows;
+  for (int c = 0; c < parts; ++c)
+    add_part(jobs, all, 32 * (full * c / parts), std::min(count, 32 * (full * (c + 1) / parts)));
+}
+
+// One warp per job: parts of 32 * rows targets (rows: 0 for the automatic choice,
+// 4 for mixed plans whose W-list surfaces carry more than 1% of the pairs, else
+// 6).  Measured on 4M points on the ellipsoid surface, NP=4, 256 per box: 2.32 ms
+// with 5 resident blocks and 4 rows against 2.50 ms with 6 and 6; uniform clouds
+// keep 6 and 6 (4.42 ms, against 4.70 ms with 4 rows).
+void add_row_jobs(const kfmm_plan* p, std::vector<P2PJob>& jobs, int rows) {
+  if (rows == 0) rows = p->prec == KFMM_MIXED && p->nf_w_heavy ? 4 : kMaxSlots;
+  for (const P2PJob& L : p->nf_leaf)
+    for (int c = 0; c < L.tcnt; c += 32 * rows) add_part(jobs, L, c, std::min(L.tcnt, c + 32 * rows));
+}
+
+// Team jobs: at most `rows` rows of 32 targets.  A
+// leaf's last row of at most 16 targets becomes a job of its own, whose warps
+// hold 2 or 4 copies of the targets and share the sources among them, when the
+// lists' entries are long enough to pay for walking them again (64 sources on
+// average; plain near field of 4M uniform points 12.25 -> 11.53 ms; with short
+// entries it loses: 4M points on the ellipsoid surface, mixed, 2.38 -> 2.54 ms).
+// Copies change the order of a target's sum, so they depend on the leaf alone.
+void add_team_jobs(const kfmm_plan* p, std::vector<P2PJob>& jobs, int rows) {
+  auto copies = [](int targets) { return targets <= 8 ? 4 : targets <= 16 ? 2 : 1; };
+  for (const P2PJob& L : p->nf_leaf) {
+    const int rem = L.tcnt % 32;
+    const bool apart = L.tcnt > 32 && rem > 0 && rem <= 16 && L.ns >= 64 * (L.eend - L.ebeg);
+    split_even(jobs, L, apart ? L.tcnt - rem : L.tcnt, rows);
+    if (apart) add_part(jobs, L, L.tcnt - rem, L.tcnt);
+    if (apart || L.tcnt <= 16) jobs.back().copies = copies(jobs.back().tcnt);
   }
+}
+
+// Whether a near field of `row_jobs` one-warp jobs runs as teams instead.  Plain
+// form: always (also at 13 jobs per resident warp, 4M uniform points, 11.97 ->
+// 11.28 ms).  Mixed form: below 4 jobs per resident warp (1M points NP 6, 2.3 jobs
+// per warp: 2.17 -> 1.92 ms; at 9, 4M points, 4.38 against 4.37 ms; at 22, the
+// ellipsoid surface, 2.26 against 2.38 ms: the longer walk's cost shows on short
+// entries).
+bool use_teams(bool mixed, size_t row_jobs, int p2p_grid) {
+  return !mixed || row_jobs < 4ull * kWarpJobsPerBlock * p2p_grid;
+}
+
+// The near field's jobs (again after a change of the tuning).
+kfmm_status build_nf_jobs(kfmm_plan* p) {
+  const int asked = p->tune.job_rows;
+  std::vector<P2PJob> jobs;
+  add_row_jobs(p, jobs, 0);  // whatever rows the tuning asks for: the sums' order stays
+  p->nf_team = use_teams(p->prec == KFMM_MIXED, jobs.size(), p->p2p_grid);
+  if (!p->nf_team && asked > 0) {
+    jobs.clear();
+    add_row_jobs(p, jobs, std::min(asked, kMaxSlots));
+  }
+  if (p->nf_team) {
+    // rows: the most, up to 4, that still give 3 jobs for every two resident teams
+    // (4,096 points: 4 rows 35 us, 2 rows 27 us)
+    const size_t want = (size_t)3 * p->num_sms *
+                        (p->prec == KFMM_MIXED ? kTeamBlocksMixed : kTeamBlocksFp64) / 2;
+    for (int rows = asked > 0 ? std::min(asked, kTeamRows) : kTeamRows; rows >= 1; --rows) {
+      jobs.clear();
+      add_team_jobs(p, jobs, rows);
+      if (jobs.size() >= want || asked > 0) break;
+    }
+  }
+  order_jobs(jobs);
   dfree(p, p->nf_jobs);
-  KF_TRY(upload(p, &p->nf_jobs, out));
-  p->n_nf = (int)out.size();
+  KF_TRY(upload(p, &p->nf_jobs, jobs));
+  p->n_nf = (int)jobs.size();
   p->nf_minb5 = p->prec == KFMM_MIXED &&
                 (p->tune.nf_blocks == 5 || (p->tune.nf_blocks == 0 && p->nf_w_heavy));
   return KFMM_OK;
@@ -550,6 +607,20 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
     int dev = 0;
     KF_CUDA(cudaGetDevice(&dev));
     KF_CUDA(cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, dev));
+  }
+  {
+    int occ = 0;
+    if (p->prec == KFMM_MIXED)
+      KF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, p2p_warp_kernel<true>,
+                                                            32 * kWarpJobsPerBlock, 0));
+    else
+      KF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, p2p_warp_kernel<false>,
+                                                            32 * kWarpJobsPerBlock, 0));
+    p->p2p_grid = std::max(1, occ) * p->num_sms;
+    int occ5 = 0;
+    KF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ5, p2p_warp_kernel<true, 5>,
+                                                          32 * kWarpJobsPerBlock, 0));
+    p->p2p_grid5 = std::max(1, occ5) * p->num_sms;
   }
   Operators op = operators_for(np);
   if (user) {
@@ -599,8 +670,10 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
     KF_TRY(upload(p, &p->ctrf, cf));
   }
   KF_TRY(upload(p, &p->d_depth, std::vector<int>(d->depth, d->depth + nn)));
-  KF_TRY(upload(p, &p->d_src_beg, std::vector<int>(d->src_beg, d->src_beg + nn)));
-  KF_TRY(upload(p, &p->d_src_num, std::vector<int>(d->src_num, d->src_num + nn)));
+  if (p->prec == KFMM_MIXED) {
+    KF_TRY(upload(p, &p->d_src_beg, std::vector<int>(d->src_beg, d->src_beg + nn)));
+    KF_TRY(upload(p, &p->d_src_num, std::vector<int>(d->src_num, d->src_num + nn)));
+  }
   KF_TRY(upload(p, &p->d_src_perm, std::vector<int>(d->src_perm, d->src_perm + d->num_src)));
   KF_TRY(upload(p, &p->d_trg_perm, std::vector<int>(d->trg_perm, d->trg_perm + d->num_trg)));
   {
@@ -735,73 +808,55 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
   KF_CUDA(cudaMemset(p->spec, 0, p->cplx * (size_t)nn * p->Fpad));
   KF_CUDA(cudaMemset(p->effv, 0, p->cplx * (size_t)nn * p->Fpad));
 
-  const int chunk = 32 * kMaxSlots;  // targets per S2M / S2L job (near field: build_nf_jobs)
-  auto add_chunks = [&](std::vector<P2PJob>& jobs, int tnode, int tkind, int tbeg0, int tcount,
-                        int ebeg, int eend, int out0, int mode) {
-    for (int c = 0; c < tcount; c += chunk) {
-      P2PJob j;
-      j.tnode = tnode;
-      j.tkind = tkind;
-      j.tbeg = tbeg0 + c;
-      j.tcnt = std::min(chunk, tcount - c);
-      j.ebeg = ebeg;
-      j.eend = eend;
-      j.out = out0 + c;
-      j.mode = mode;
-      jobs.push_back(j);
-    }
+  // one entry: the sources of leaf `node`, or (kind 1, 2) its UE or DE surface
+  auto entry = [&](int kind, int node) {
+    return kind == 0 ? P2PEntry{d->src_beg[node], d->src_num[node], 0, node}
+                     : P2PEntry{0, P, kind, node};
   };
-  auto src_count = [&](int ent) -> int {
-    int kind = ent >> 28, node = ent & 0x0fffffff;
-    return kind == 0 ? d->src_num[node] : P;
+  auto ids_of = [](const std::vector<P2PEntry>& ent) {
+    std::vector<int> ids(ent.size());
+    for (size_t k = 0; k < ent.size(); ++k) ids[k] = ent[k].kind << 28 | ent[k].node;
+    return ids;
   };
-  // For the persistent P2P kernel: largest first, by cost class (target slots
-  // x sources, in classes 5% wide); within a class the jobs keep their tree
-  // order, so warps working at the same time read neighbouring leaves' sources
-  // and the L2 cache serves the repeats.
-  auto order_jobs = [&](std::vector<P2PJob>& jobs, const std::vector<int>& ent,
-                        std::vector<float>* class_out = nullptr) {
-    std::vector<std::pair<double, int>> key(jobs.size());
-    for (size_t j = 0; j < jobs.size(); ++j) {
-      double ns = 0;
-      for (int k = jobs[j].ebeg; k < jobs[j].eend; ++k) ns += src_count(ent[k]);
-      const double cost = std::max(1.0, ns * ((jobs[j].tcnt + 31) / 32));
-      key[j] = {-std::floor(std::log(cost) / std::log(kCostClassWidth)), (int)j};
+  // uploads a list's entries in the form the plan's row jobs read
+  auto upload_entries = [&](const std::vector<P2PEntry>& ent, P2PEntry** e, int** ids) {
+    return p->prec == KFMM_MIXED ? upload(p, ids, ids_of(ent)) : upload(p, e, ent);
+  };
+  // Check-surface jobs (S2M, S2L; one warp each): the most rows of targets, up to
+  // 6, that still give 3 jobs for every two resident warps (S2M, plain: 65,536
+  // points NP 4 47 -> 27 us; 1M points NP 6 stays at 5 rows).
+  auto split_jobs = [&](const std::vector<P2PJob>& all, std::vector<P2PJob>& jobs) {
+    const size_t want = (size_t)3 * kWarpJobsPerBlock * p->p2p_grid / 2;
+    for (int rows = kMaxSlots; rows >= 1; --rows) {
+      jobs.clear();
+      for (const P2PJob& j : all) split_even(jobs, j, j.tcnt, rows);
+      if (jobs.size() >= want) break;
     }
-    std::stable_sort(key.begin(), key.end(),
-                     [](const std::pair<double, int>& a, const std::pair<double, int>& b) {
-                       return a.first < b.first;
-                     });
-    std::vector<P2PJob> out(jobs.size());
-    for (size_t j = 0; j < jobs.size(); ++j) out[j] = jobs[key[j].second];
-    jobs.swap(out);
-    if (class_out) {
-      class_out->resize(jobs.size());
-      for (size_t j = 0; j < jobs.size(); ++j) (*class_out)[j] = (float)key[j].first;
-    }
+    order_jobs(jobs);
   };
 
   // --- up: S2M jobs + UC2UE GEMM, then M2M per level
   {
-    std::vector<P2PJob> jobs;
-    std::vector<int> ent, boff, coff;
+    std::vector<P2PJob> all, jobs;
+    std::vector<P2PEntry> ent;
+    std::vector<int> boff, coff;
     std::vector<double> alpha;
     int slot = 0;
     for (int i = 0; i < nn; ++i) {
       if (!is_leaf(i) || !has_src(i)) continue;
-      int e = (int)ent.size();
-      ent.push_back(i);
-      add_chunks(jobs, i, 1, 0, Q, e, e + 1, slot * Q, 0);
+      const int e = (int)ent.size();
+      ent.push_back(entry(0, i));
+      all.push_back(P2PJob{i, 1, 0, Q, e, e + 1, slot * Q, 0, d->src_num[i]});
       p->stats.s2m_pairs += (double)Q * d->src_num[i];
       boff.push_back(slot * Q);
       coff.push_back(i * P);
       alpha.push_back(std::ldexp(1.0, -d->depth[i]));
       ++slot;
     }
-    order_jobs(jobs, ent);
+    split_jobs(all, jobs);
     p->n_s2m = (int)jobs.size();
     KF_TRY(upload(p, &p->s2m_jobs, jobs));
-    KF_TRY(upload(p, &p->s2m_ent, ent));
+    KF_TRY(upload_entries(ent, &p->s2m_ent, &p->s2m_ids));
     KF_TRY(dalloc(p, &p->chk_up, (size_t)std::max(slot, 1) * Q));
     KF_TRY(add_gemm(p, p->up_gemms, p->d_uc2ue, P, Q, p->chk_up, boff, p->uden, coff, &alpha, 0, 0));
     int maxpar = 1;
@@ -1061,8 +1116,8 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
 
   // --- X list S2L jobs
   {
-    std::vector<P2PJob> jobs;
-    std::vector<int> ent;
+    std::vector<P2PJob> all, jobs;
+    std::vector<P2PEntry> ent;
     for (int t = 0; t < nn; ++t) {
       if (!has_trg(t)) continue;
       int xb = d->x_ptr[t], xe = d->x_ptr[t + 1];
@@ -1071,16 +1126,16 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
       int e0 = (int)ent.size();
       int ns = 0;
       for (int k = xb; k < xe; ++k) {
-        ent.push_back(d->x_idx[k]);
+        if (d->src_num[d->x_idx[k]] > 0) ent.push_back(entry(0, d->x_idx[k]));
         ns += d->src_num[d->x_idx[k]];
       }
-      add_chunks(jobs, t, 2, 0, P, e0, (int)ent.size(), t * P, 1);
+      all.push_back(P2PJob{t, 2, 0, P, e0, (int)ent.size(), t * P, 1, ns});
       p->stats.s2l_pairs += (double)P * ns;
     }
-    order_jobs(jobs, ent);
+    split_jobs(all, jobs);
     p->n_s2l = (int)jobs.size();
     KF_TRY(upload(p, &p->s2l_jobs, jobs));
-    KF_TRY(upload(p, &p->s2l_ent, ent));
+    KF_TRY(upload_entries(ent, &p->s2l_ent, &p->s2l_ids));
   }
 
   // --- down: L2L per level
@@ -1104,8 +1159,7 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
 
   // --- near field: U + W + direct X + L2T
   {
-    std::vector<P2PJob> jobs;
-    std::vector<int> ent;
+    std::vector<P2PEntry> ent;
     // Pairs with W-list UE surfaces: where they carry more than 1% of the
     // pairs (clouds on surfaces), the mixed near field runs with 5 resident
     // blocks per SM and jobs of at most 4 rows (128 targets): measured on 4M
@@ -1171,33 +1225,49 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
     for (int t = 0; t < nn; ++t) {
       if (!is_leaf(t) || !has_trg(t) || d->trg_num[t] == 0) continue;
       int e0 = (int)ent.size();
-      for (int k = d->u_ptr[t]; k < d->u_ptr[t + 1]; ++k) ent.push_back(d->u_idx[k]);
+      for (int k = d->u_ptr[t]; k < d->u_ptr[t + 1]; ++k) ent.push_back(entry(0, d->u_idx[k]));
       const int e_after_u = (int)ent.size();
       for (int k = d->w_ptr[t]; k < d->w_ptr[t + 1]; ++k) {
         int s = d->w_idx[k];
         bool direct = is_leaf(s) && d->src_num[s] < P;  // fmm/omp.cc:675
-        ent.push_back(direct ? s : ((1 << 28) | s));
+        ent.push_back(entry(direct ? 0 : 1, s));
       }
       if (d->trg_num[t] < P)  // fmm/omp.cc:724
-        for (int k = d->x_ptr[t]; k < d->x_ptr[t + 1]; ++k) ent.push_back(d->x_idx[k]);
-      if (d->depth[t] >= 2) ent.push_back((2 << 28) | t);
+        for (int k = d->x_ptr[t]; k < d->x_ptr[t + 1]; ++k)
+          ent.push_back(entry(0, d->x_idx[k]));
+      if (d->depth[t] >= 2) ent.push_back(entry(2, t));
       if (on_host[t]) e0 = e_after_u;  // the host sums this leaf's U list
+      // entries without sources leave the list; the plain form's points carry
+      // absolute coordinates, so ranges that touch become one (but not with the
+      // leaf's own, whose pairs may coincide)
+      std::vector<P2PEntry> list(ent.begin() + e0, ent.end());
+      list.erase(std::remove_if(list.begin(), list.end(),
+                                [](const P2PEntry& q) { return q.count == 0; }),
+                 list.end());
+      if (p->prec != KFMM_MIXED) {
+        std::stable_sort(list.begin(), list.end(), [](const P2PEntry& a, const P2PEntry& b) {
+          return a.kind != b.kind ? a.kind < b.kind : a.kind == 0 && a.base < b.base;
+        });
+        size_t m = 0;
+        for (size_t k = 0; k < list.size(); ++k) {
+          if (m > 0 && list[k].kind == 0 && list[k].node != t && list[m - 1].node != t &&
+              list[m - 1].base + list[m - 1].count == list[k].base)
+            list[m - 1].count += list[k].count;
+          else
+            list[m++] = list[k];
+        }
+        list.resize(m);
+      }
+      ent.resize(e0);
+      ent.insert(ent.end(), list.begin(), list.end());
       int ns = 0;
-      for (int k = e0; k < (int)ent.size(); ++k) ns += src_count(ent[k]);
-      P2PJob j;
-      j.tnode = t;
-      j.tkind = 0;
-      j.tbeg = d->trg_beg[t];
-      j.tcnt = d->trg_num[t];
-      j.ebeg = e0;
-      j.eend = (int)ent.size();
-      j.out = d->trg_beg[t];
-      j.mode = 0;
-      p->nf_leaf.push_back(j);
-      p->nf_leaf_ns.push_back(ns);
+      for (const P2PEntry& q : list) ns += q.count;
+      p->nf_leaf.push_back(P2PJob{t, 0, d->trg_beg[t], d->trg_num[t], e0, (int)ent.size(),
+                                  d->trg_beg[t], 0, ns});
       p->stats.u_pairs += (double)d->trg_num[t] * ns;
     }
     KF_TRY(upload(p, &p->nf_ent, ent));
+    if (p->prec == KFMM_MIXED) KF_TRY(upload(p, &p->nf_ids, ids_of(ent)));
     KF_TRY(build_nf_jobs(p));
   }
 
@@ -1219,20 +1289,6 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
   KF_TRY(dalloc(p, &p->job_counter, 3));
   KF_TRY(dalloc(p, &p->d_error, 2));
   KF_CUDA(cudaMemset(p->d_error, 0, 2 * sizeof(int)));
-  {
-    int occ = 0;
-    if (p->prec == KFMM_MIXED)
-      KF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, p2p_warp_kernel<true>,
-                                                            32 * kWarpJobsPerBlock, 0));
-    else
-      KF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, p2p_warp_kernel<false>,
-                                                            32 * kWarpJobsPerBlock, 0));
-    p->p2p_grid = std::max(1, occ) * p->num_sms;
-    int occ5 = 0;
-    KF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ5, p2p_warp_kernel<true, 5>,
-                                                          32 * kWarpJobsPerBlock, 0));
-    p->p2p_grid5 = std::max(1, occ5) * p->num_sms;
-  }
   p->stats.num_nodes = nn;
   p->stats.P = P;
   p->stats.Q = Q;
@@ -1311,20 +1367,29 @@ kfmm_status launch_fft(int np, bool mixed, bool forward, int nboxes, int num_sms
 }
 
 kfmm_status launch_p2p(const kfmm_plan* p, int which, int njobs, const P2PParams& q,
-                       void* stream, const char* what) {
-  const int blocks = std::min(p->p2p_grid, (njobs + kWarpJobsPerBlock - 1) / kWarpJobsPerBlock);
-  int* counter = p->job_counter + which;
-  KF_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), S(stream)));
-  if (p->prec == KFMM_MIXED && which == 2 && p->nf_minb5)
-    p2p_warp_kernel<true, 5><<<std::min(p->p2p_grid5, (njobs + kWarpJobsPerBlock - 1) /
-                                                          kWarpJobsPerBlock),
-                               32 * kWarpJobsPerBlock, 0, S(stream)>>>(
-        p2p_mixed_params(p, q, p->d_trg_perm), njobs, counter);
-  else if (p->prec == KFMM_MIXED)
-    p2p_warp_kernel<true><<<blocks, 32 * kWarpJobsPerBlock, 0, S(stream)>>>(
-        p2p_mixed_params(p, q, which == 2 ? p->d_trg_perm : nullptr), njobs, counter);
-  else
-    p2p_warp_kernel<false><<<blocks, 32 * kWarpJobsPerBlock, 0, S(stream)>>>(q, njobs, counter);
+                       const int* ids, void* stream, const char* what) {
+  const bool mixed = p->prec == KFMM_MIXED;
+  const int* perm = which == 2 ? p->d_trg_perm : nullptr;
+  if (which == 2 && p->nf_team) {
+    if (mixed)
+      p2p_team_kernel<true><<<njobs, 32 * kTeam, 0, S(stream)>>>(p2p_mixed_params(p, q, ids, perm));
+    else
+      p2p_team_kernel<false><<<njobs, 32 * kTeam, 0, S(stream)>>>(q);
+  } else {
+    const bool five = which == 2 && p->nf_minb5;
+    const int blocks = std::min(five ? p->p2p_grid5 : p->p2p_grid,
+                                (njobs + kWarpJobsPerBlock - 1) / kWarpJobsPerBlock);
+    int* counter = p->job_counter + which;
+    KF_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), S(stream)));
+    if (!mixed)
+      p2p_warp_kernel<false><<<blocks, 32 * kWarpJobsPerBlock, 0, S(stream)>>>(q, njobs, counter);
+    else if (five)
+      p2p_warp_kernel<true, 5><<<blocks, 32 * kWarpJobsPerBlock, 0, S(stream)>>>(
+          p2p_mixed_params(p, q, ids, perm), njobs, counter);
+    else
+      p2p_warp_kernel<true><<<blocks, 32 * kWarpJobsPerBlock, 0, S(stream)>>>(
+          p2p_mixed_params(p, q, ids, perm), njobs, counter);
+  }
   KF_CHECK_LAUNCH(std::string("p2p kernel (") + what + ")");
   return KFMM_OK;
 }
@@ -1497,8 +1562,8 @@ kfmm_status kfmm_up_calc(kfmm_plan* p, void* stream) {
     return KFMM_ERR_STATE;
   }
   if (p->n_s2m) {
-    KF_TRY(launch_p2p(p, 0, p->n_s2m, p2p_params(p, p->s2m_jobs, p->s2m_ent, p->chk_up), stream,
-                      "s2m"));
+    KF_TRY(launch_p2p(p, 0, p->n_s2m, p2p_params(p, p->s2m_jobs, p->s2m_ent, p->chk_up),
+                      p->s2m_ids, stream, "s2m"));
   }
   mark(p, 1, S(stream));
   return launch_gemms(p, p->up_gemms, S(stream));
@@ -1572,8 +1637,8 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
 kfmm_status kfmm_xlist_calc(kfmm_plan* p, void* stream) {
   if (!p) return KFMM_ERR_INVALID;
   if (p->n_s2l) {
-    KF_TRY(launch_p2p(p, 1, p->n_s2l, p2p_params(p, p->s2l_jobs, p->s2l_ent, p->dchk), stream,
-                      "s2l"));
+    KF_TRY(launch_p2p(p, 1, p->n_s2l, p2p_params(p, p->s2l_jobs, p->s2l_ent, p->dchk), p->s2l_ids,
+                      stream, "s2l"));
   }
   return KFMM_OK;
 }
@@ -1591,7 +1656,7 @@ kfmm_status near_field(kfmm_plan* p, void* stream) {
   }
   if (p->n_nf) {
     KF_TRY(launch_p2p(p, 2, p->n_nf, p2p_params(p, p->nf_jobs, p->nf_ent, near_field_out(p)),
-                      stream, "near field"));
+                      p->nf_ids, stream, "near field"));
   }
   return KFMM_OK;
 }
@@ -1902,10 +1967,10 @@ struct kfmm_batch {
   std::vector<cudaEvent_t> events;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  // fused near field of all plans: per-plan kernel arguments, (plan, job)
-  // pairs in cost-class order, the job counter
+  // fused near field of all plans: per-plan kernel arguments, all jobs in
+  // cost-class order, the job counter
   void* d_params = nullptr;  // P2PMixedParams (mixed plans) or P2PParams
-  int2* d_jobs = nullptr;
+  P2PJob* d_jobs = nullptr;  // team jobs, then one-warp jobs
   int* d_counter = nullptr;
   std::vector<kfmm_plan*> plans;  // for the error flags kfmm_batch_wait reads
 };
@@ -1957,48 +2022,53 @@ kfmm_status kfmm_batch_create(kfmm_plan* const* plans, int nplans, int nstreams,
     if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
       return fail(e, "cudaEventCreate");
   }
-  // Plans of one precision share one near-field launch: their far fields run
+  // Plans of one precision share their near-field launches: their far fields run
   // on the branch streams, then a single persistent launch takes the jobs of
   // all plans, largest cost class first, so small solves do not leave SMs
   // idle.
+  const bool mixed = plans[0]->prec == KFMM_MIXED;
   bool fused = true;
-  size_t njobs = 0;
-  for (int i = 0; i < nplans; ++i) {
-    fused = fused && plans[i]->prec == plans[0]->prec;
-    njobs += plans[i]->n_nf;
-  }
-  fused = fused && njobs > 0 && njobs < (size_t)INT32_MAX;
+  for (int i = 0; i < nplans; ++i) fused = fused && plans[i]->prec == plans[0]->prec;
   // A single solve is captured as its own launches (its near field keeps the
   // by-value argument block of the regular kernel).
   const bool single = nplans == 1;
   if (single) fused = false;
+  // Each plan's jobs are of the kind its own solve has, so a replay gives the same
+  // bits; team jobs have the most rows, as the plans fill the device together.
+  std::vector<P2PJob> jobs, row_jobs;
   if (fused) {
-    const bool mixed = plans[0]->prec == KFMM_MIXED;
+    for (int i = 0; i < nplans; ++i) {
+      const kfmm_plan* p = plans[i];
+      const int asked = p->tune.job_rows;
+      std::vector<P2PJob>& to = p->nf_team ? jobs : row_jobs;
+      const size_t from = to.size();
+      if (p->nf_team) add_team_jobs(p, to, asked > 0 ? std::min(asked, kTeamRows) : kTeamRows);
+      else add_row_jobs(p, to, asked > 0 ? std::min(asked, kMaxSlots) : 0);
+      for (size_t j = from; j < to.size(); ++j) to[j].plan = i;
+    }
+    fused = jobs.size() + row_jobs.size() > 0 && jobs.size() + row_jobs.size() < (size_t)INT32_MAX;
+  }
+  const int nteam = (int)jobs.size(), nrow = (int)row_jobs.size();
+  if (fused) {
+    order_jobs(jobs);
+    order_jobs(row_jobs);
+    jobs.insert(jobs.end(), row_jobs.begin(), row_jobs.end());
     std::vector<P2PParams> params(nplans);
     std::vector<P2PMixedParams> mparams(mixed ? nplans : 0);
-    std::vector<std::pair<float, int2>> order;
-    order.reserve(njobs);
     for (int i = 0; i < nplans; ++i) {
       kfmm_plan* p = plans[i];
       params[i] = p2p_params(p, p->nf_jobs, p->nf_ent, near_field_out(p));
-      if (mixed) mparams[i] = p2p_mixed_params(p, params[i], p->d_trg_perm);
-      for (int j = 0; j < p->n_nf; ++j) order.push_back({p->nf_class[j], make_int2(i, j)});
+      if (mixed) mparams[i] = p2p_mixed_params(p, params[i], p->nf_ids, p->d_trg_perm);
     }
-    std::stable_sort(order.begin(), order.end(),
-                     [](const std::pair<float, int2>& a, const std::pair<float, int2>& c) {
-                       return a.first < c.first;
-                     });
-    std::vector<int2> jobs(njobs);
-    for (size_t j = 0; j < njobs; ++j) jobs[j] = order[j].second;
     const size_t pbytes = mixed ? sizeof(P2PMixedParams) * nplans : sizeof(P2PParams) * nplans;
     const void* psrc = mixed ? (const void*)mparams.data() : (const void*)params.data();
+    const size_t jbytes = sizeof(P2PJob) * jobs.size();
     if ((e = cudaMalloc(&b->d_params, pbytes)) != cudaSuccess ||
-        (e = cudaMalloc(&b->d_jobs, sizeof(int2) * njobs)) != cudaSuccess ||
+        (e = cudaMalloc(&b->d_jobs, jbytes)) != cudaSuccess ||
         (e = cudaMalloc(&b->d_counter, sizeof(int))) != cudaSuccess)
       return fail(e, "cudaMalloc");
     if ((e = cudaMemcpy(b->d_params, psrc, pbytes, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(b->d_jobs, jobs.data(), sizeof(int2) * njobs, cudaMemcpyHostToDevice)) !=
-            cudaSuccess)
+        (e = cudaMemcpy(b->d_jobs, jobs.data(), jbytes, cudaMemcpyHostToDevice)) != cudaSuccess)
       return fail(e, "cudaMemcpy");
   }
   cudaStream_t origin = b->streams[nstreams];
@@ -2026,15 +2096,19 @@ kfmm_status kfmm_batch_create(kfmm_plan* const* plans, int nplans, int nstreams,
   }
   if (!single) join();
   if (fused && st == KFMM_OK) {
-    cudaMemsetAsync(b->d_counter, 0, sizeof(int), origin);
-    const int blocks = std::min(plans[0]->p2p_grid,
-                                (int)((njobs + kWarpJobsPerBlock - 1) / kWarpJobsPerBlock));
-    if (plans[0]->prec == KFMM_MIXED)
-      p2p_fused_kernel<true><<<blocks, 32 * kWarpJobsPerBlock, 0, origin>>>(
-          (const P2PMixedParams*)b->d_params, b->d_jobs, (int)njobs, b->d_counter);
-    else
-      p2p_fused_kernel<false><<<blocks, 32 * kWarpJobsPerBlock, 0, origin>>>(
-          (const P2PParams*)b->d_params, b->d_jobs, (int)njobs, b->d_counter);
+    if (nteam && mixed)
+      p2p_team_batch_kernel<true><<<nteam, 32 * kTeam, 0, origin>>>(
+          (const P2PMixedParams*)b->d_params, b->d_jobs);
+    else if (nteam)
+      p2p_team_batch_kernel<false><<<nteam, 32 * kTeam, 0, origin>>>((const P2PParams*)b->d_params,
+                                                                     b->d_jobs);
+    if (nrow) {  // mixed plans only
+      cudaMemsetAsync(b->d_counter, 0, sizeof(int), origin);
+      const int blocks =
+          std::min(plans[0]->p2p_grid, (nrow + kWarpJobsPerBlock - 1) / kWarpJobsPerBlock);
+      p2p_fused_kernel<<<blocks, 32 * kWarpJobsPerBlock, 0, origin>>>(
+          (const P2PMixedParams*)b->d_params, b->d_jobs + nteam, nrow, b->d_counter);
+    }
     if (cudaGetLastError() != cudaSuccess) {
       set_error("kfmm_batch_create: fused near-field launch failed");
       st = KFMM_ERR_CUDA;
