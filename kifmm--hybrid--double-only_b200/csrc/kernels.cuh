@@ -1345,121 +1345,20 @@ __global__ void __launch_bounds__(kFFTThreads) ifft_trg_np_kernel(FFTParams p) {
 // = (wx + 6 wy + 36 wz); member c = 4 cx + 2 cy + cz; offset delta = w - 2 -
 // (cx,cy,cz) selects translation spectrum (dx+3) + 7 (dy+3) + 49 (dz+3)
 // (fmm/omp_sse_block.cc:581-593).
-struct HadamardParams {
-  int nn, ngroups, groups_per_block;
-  const int* win;      // ngroups x 216 node ids (-1 = absent)
-  const int* members;  // ngroups x 8 node ids (-1 = no V list)
-  // 343 x Fpad translation spectra, zero for |delta|_inf <= 1 and f >= F
-  const double2* trans;
-  int Fpad;
-  const double2* spec;  // blocked layout
-  double2* effv;        // blocked layout
-};
-
-constexpr int kHadThreads = 256;  // 8 warps, one group per warp, lane = frequency
-constexpr int kHadGroupsInFlight = kHadThreads / 32;
-constexpr int kHadGroupsPerBlock = 32;
+// Spectra in blocks of kFB = 32 frequencies, lane = frequency.  A window's rows in
+// x meet, for each of the 4 (cy, cz) member pairs, one row of 7 translation
+// spectra.  Pairs of sibling groups whose parents are x-neighbours (parent x even
+// and x + 1) share one 8 x 6 x 6 window, so each translation value serves both.
+constexpr int kHadMaxWin = 288;  // 8 x 6 x 6
 
 // A row of the translation table at (dy, dz) with |dy| <= 1 and |dz| <= 1:
 // its entries dx = -1, 0, 1 (k = 2, 3, 4 of the row) are adjacent offsets,
 // whose spectra are zero (they are not V-list interactions), so the FP64
-// window kernel skips those loads and multiply-adds: 27 of the 216 per member.
+// kernel skips those loads and multiply-adds: 27 of the 216 per member.
 // (The FP32 kernels below are FMA-bound with their loads scheduled across the
 // rows; there a branch per row costs more than the skipped work.)
 __device__ __forceinline__ bool near_row(int dy, int dz) {
   return dy >= -1 && dy <= 1 && dz >= -1 && dz <= 1;
-}
-
-__device__ __forceinline__ void cmac64(double& ar, double& ai, const double2 t, const double2 s) {
-  ar = fma(t.x, s.x, ar);
-  ar = fma(-t.y, s.y, ar);
-  ai = fma(t.x, s.y, ai);
-  ai = fma(t.y, s.x, ai);
-}
-
-// Plain FP64 form.  One block: one block of 32 frequencies (blockIdx.y) for
-// groups_per_block groups.  Warp = one group, lane = one frequency, all 8
-// members of the group in registers; every load of a warp is 32 distinct,
-// contiguous values.  The translation spectra are read through L1 (the
-// frequency block's FP64 tile, 176 KB, would leave room for one block per
-// SM).  The window is walked row by row in x: a row of 6 source spectra
-// meets, for each of the 4 (cy, cz) member pairs, one row of 7 translation
-// spectra: 12 complex multiply-adds per 7 loads; the next row's source
-// spectra are fetched while the current row is multiplied.
-__global__ void __launch_bounds__(kHadThreads) hadamard_kernel(HadamardParams p) {
-  __shared__ int win[kHadGroupsInFlight][216];
-  __shared__ int mem[kHadGroupsInFlight][8];
-  const int fb = blockIdx.y;
-  const int f = threadIdx.x & 31, slot = threadIdx.x >> 5;
-  const int g0 = blockIdx.x * p.groups_per_block;
-  const int g1 = min(p.ngroups, g0 + p.groups_per_block);
-  const size_t fbase = (size_t)fb * p.nn;
-  for (int gb = g0; gb < g1; gb += kHadGroupsInFlight) {
-    __syncthreads();
-    for (int q = threadIdx.x; q < kHadGroupsInFlight * 216; q += kHadThreads) {
-      const int g = gb + q / 216;
-      win[q / 216][q % 216] = g < g1 ? p.win[(size_t)g * 216 + q % 216] : -1;
-    }
-    for (int q = threadIdx.x; q < kHadGroupsInFlight * 8; q += kHadThreads) {
-      const int g = gb + q / 8;
-      mem[q / 8][q % 8] = g < g1 ? p.members[(size_t)g * 8 + q % 8] : -1;
-    }
-    __syncthreads();
-    if (gb + slot >= g1) continue;  // warp-uniform: no group for this warp
-    const int* w = win[slot];
-    double2 nxt[6];
-#pragma unroll
-    for (int wx = 0; wx < 6; ++wx) {
-      const int sid = w[wx];
-      nxt[wx] = sid >= 0 ? p.spec[(fbase + sid) * kFB + f] : make_double2(0.0, 0.0);
-    }
-    double ar[8], ai[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) ar[c] = ai[c] = 0.0;
-    for (int row = 0; row < 36; ++row) {
-      double2 srow[6];
-#pragma unroll
-      for (int wx = 0; wx < 6; ++wx) srow[wx] = nxt[wx];
-      if (row + 1 < 36) {
-#pragma unroll
-        for (int wx = 0; wx < 6; ++wx) {
-          const int sid = w[(row + 1) * 6 + wx];
-          nxt[wx] = sid >= 0 ? p.spec[(fbase + sid) * kFB + f] : make_double2(0.0, 0.0);
-        }
-      }
-      const int wy = row % 6, wz = row / 6;
-#pragma unroll
-      for (int cyz = 0; cyz < 4; ++cyz) {
-        const int cy = cyz >> 1, cz = cyz & 1;
-        const double2* trow =
-            p.trans + (size_t)((wz - 2 - cz + 3) * 49 + (wy - 2 - cy + 3) * 7) * p.Fpad +
-            fb * kFB + f;
-        auto row_body = [&](auto near) {
-          constexpr bool kNear = decltype(near)::value;
-          double2 t[7];
-#pragma unroll
-          for (int k = 0; k < 7; ++k)
-            t[k] = kNear && k >= 2 && k <= 4 ? make_double2(0.0, 0.0)
-                                            : __ldg(trow + (size_t)k * p.Fpad);
-#pragma unroll
-          for (int wx = 0; wx < 6; ++wx)
-#pragma unroll
-            for (int cx = 0; cx < 2; ++cx) {
-              const int c = cx * 4 + cy * 2 + cz, k = wx - cx + 1;
-              if (kNear && k >= 2 && k <= 4) continue;
-              cmac64(ar[c], ai[c], t[k], srow[wx]);
-            }
-        };
-        if (near_row(wy - 2 - cy, wz - 2 - cz)) row_body(std::true_type{});
-        else row_body(std::false_type{});
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const int m = mem[slot][c];
-      if (m >= 0) p.effv[(fbase + m) * kFB + f] = make_double2(ar[c], ai[c]);
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1479,7 +1378,7 @@ __global__ void __launch_bounds__(kHadThreads) hadamard_kernel(HadamardParams p)
 constexpr int kHad32Threads = 512;
 constexpr int kHad32Warps = kHad32Threads / 32;
 constexpr unsigned kHad32TileBytes = 343u * kFB * 8u;  // 87,808
-constexpr int kHad32Copies = 7;                         // 49 offsets (12,544 B) each
+constexpr int kHadCopies = 7;                           // 49 offsets each
 constexpr long long kMbarSpinLimit = 1ll << 24;          // bounded waits
 
 struct Had32Params {
@@ -1512,14 +1411,15 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned bar, unsigned parity,
   return false;
 }
 
-// Bulk-copies the translation tile of frequency block fb into dst (one
-// thread issues, all wait on the mbarrier with a bounded spin of `limit`
+// Bulk-copies kBytes of a translation tile from src into dst in 7 copies of 49
+// offsets (one thread issues, all wait on the mbarrier with a bounded spin of `limit`
 // tries).  Returns false in every thread of the block, after setting *error,
 // if the copy did not complete; thread 0 then waits (with the full default
 // bound) for the copy still in flight to land before the block exits.
-__device__ __forceinline__ bool had32_load_tile(const float2* tile, int fb, unsigned char* dst,
-                                                unsigned long long* bar, int* error,
-                                                long long limit) {
+template <unsigned kBytes>
+__device__ __forceinline__ bool had_load_tile(const void* tile, unsigned char* dst,
+                                              unsigned long long* bar, int* error,
+                                              long long limit) {
   const unsigned b = smem_addr(bar);
   if (threadIdx.x == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(b) : "memory");
@@ -1529,12 +1429,12 @@ __device__ __forceinline__ bool had32_load_tile(const float2* tile, int fb, unsi
   __syncthreads();
   if (threadIdx.x == 0) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(b),
-                 "r"(kHad32TileBytes)
+                 "r"(kBytes)
                  : "memory");
-    const unsigned char* src = (const unsigned char*)(tile + (size_t)fb * 343 * kFB);
-    constexpr unsigned chunk = kHad32TileBytes / kHad32Copies;
+    const unsigned char* src = (const unsigned char*)tile;
+    constexpr unsigned chunk = kBytes / kHadCopies;
 #pragma unroll 1
-    for (int c = 0; c < kHad32Copies; ++c)
+    for (int c = 0; c < kHadCopies; ++c)
       asm volatile(
           "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, "
           "[%3];\n" ::"r"(smem_addr(dst + c * chunk)),
@@ -1552,6 +1452,145 @@ __device__ __forceinline__ bool had32_load_tile(const float2* tile, int fb, unsi
   return true;
 }
 
+// Plain FP64 form, one CTA per SM: the frequency block's 343 translation spectra
+// (175,616 B) are brought into shared memory by bulk asynchronous copies, a warp
+// takes one window of H sibling groups (H = 2: an x-pair), all 8 H members'
+// sums in registers.  Bound by the FP64 pipe: a row of H = 2 is 384 multiply-adds
+// a lane (192 cycles of the SM's pipe) against 112 shared-memory wavefronts of
+// translation values and 32 of sources; with one group a window the wavefronts
+// outweighed the multiply-adds.
+// Where there are fewer windows than warps on the device, `split` warps share a
+// window, each taking every split-th of its rows; their sums meet in shared
+// memory (over the tile, once every warp is done with it) and are added in order.
+constexpr int kHad64Threads = 256;
+constexpr int kHad64Warps = kHad64Threads / 32;
+constexpr unsigned kHad64TileBytes = 343u * kFB * 16u;  // 175,616
+
+struct Had64Params {
+  int nn, nwin, win_per_block, split;
+  const int* win;      // nwin x (4 + 2H) x 6 x 6 node ids, x fastest (-1 = absent)
+  const int* members;  // nwin x 8H node ids (-1 = no V list)
+  const unsigned long long* rows;  // per window: bit wy + 6 wz set if the row has an entry
+  const double2* tile;  // [fb][343][32], zero for |delta|_inf <= 1 and f >= F
+  const double2* spec;
+  double2* effv;
+  int* error;  // set to 1 when the tile copy does not complete
+};
+
+template <int H>
+__global__ void __launch_bounds__(kHad64Threads, 1) hadamard_fp64_kernel(Had64Params p) {
+  constexpr int WX = 4 + 2 * H, C = 8 * H;
+  extern __shared__ __align__(128) unsigned char had32_dyn[];
+  __shared__ int win[kHad64Warps][36 * WX];
+  __shared__ int mem[kHad64Warps][C];
+  __shared__ __align__(8) unsigned long long bar;
+  const double2* tsm = (const double2*)had32_dyn;
+  const int fb = blockIdx.y;
+  const int f = threadIdx.x & 31, slot = threadIdx.x >> 5;
+  const int teams = kHad64Warps / p.split, part = slot % p.split;
+  const int g0 = blockIdx.x * p.win_per_block;
+  const int g1 = min(p.nwin, g0 + p.win_per_block);
+  const size_t fbase = (size_t)fb * p.nn;
+  const double2* spec = p.spec + fbase * kFB + f;
+  if (!had_load_tile<kHad64TileBytes>(p.tile + (size_t)fb * 343 * kFB, had32_dyn, &bar, p.error,
+                                      kMbarSpinLimit))
+    return;
+  unsigned long long mine = ~0ull;  // this warp's rows of a window
+  if (p.split > 1) {
+    mine = 0ull;
+    for (int r = part; r < 36; r += p.split) mine |= 1ull << r;
+  }
+  double ar[C], ai[C];
+  for (int g = g0 + slot / p.split; g < g1; g += teams) {
+    for (int q = f; q < 36 * WX; q += 32) win[slot][q] = p.win[(size_t)g * (36 * WX) + q];
+    if (f < C) mem[slot][f] = p.members[(size_t)g * C + f];
+    __syncwarp();
+    const int* w = win[slot];
+    unsigned long long rows = p.rows[g] & mine;
+#pragma unroll
+    for (int c = 0; c < C; ++c) ar[c] = ai[c] = 0.0;
+    double2 nxt[WX];
+    auto fetch = [&](int r) {
+#pragma unroll
+      for (int x = 0; x < WX; ++x) {
+        const int sid = w[r * WX + x];
+        nxt[x] = sid >= 0 ? spec[(size_t)sid * kFB] : make_double2(0.0, 0.0);
+      }
+    };
+    int row = rows ? __ffsll((long long)rows) - 1 : 36;
+    if (row < 36) fetch(row);
+    while (row < 36) {
+      rows &= rows - 1;
+      const int next = rows ? __ffsll((long long)rows) - 1 : 36;
+      double2 srow[WX];
+#pragma unroll
+      for (int x = 0; x < WX; ++x) srow[x] = nxt[x];
+      if (next < 36) fetch(next);
+      const int wy = row % 6, wz = row / 6;
+#pragma unroll
+      for (int cyz = 0; cyz < 4; ++cyz) {
+        const int cy = cyz >> 1, cz = cyz & 1;
+        const double2* trow = tsm + ((wz + 1 - cz) * 49 + (wy + 1 - cy) * 7) * kFB + f;
+        auto row_body = [&](auto near) {
+          constexpr bool kNear = decltype(near)::value;
+#pragma unroll
+          for (int k = 0; k < 7; ++k) {
+            if (kNear && k >= 2 && k <= 4) continue;
+            const double2 t = trow[k * kFB];
+            // the products with t.x of all members first, then those with t.y: the
+            // two a sum receives are then 2 H x 2 operations apart, not adjacent
+#pragma unroll
+            for (int part = 0; part < 2; ++part)
+#pragma unroll
+              for (int h = 0; h < H; ++h)
+#pragma unroll
+                for (int cx = 0; cx < 2; ++cx) {
+                  const int wx = k - 1 + cx;
+                  if (wx < 0 || wx > 5) continue;
+                  const int c = h * 8 + cx * 4 + cy * 2 + cz;
+                  const double2 v = srow[wx + 2 * h];
+                  ar[c] = part == 0 ? fma(t.x, v.x, ar[c]) : fma(-t.y, v.y, ar[c]);
+                  ai[c] = part == 0 ? fma(t.x, v.y, ai[c]) : fma(t.y, v.x, ai[c]);
+                }
+          }
+        };
+        if (near_row(wy - 2 - cy, wz - 2 - cz)) row_body(std::true_type{});
+        else row_body(std::false_type{});
+      }
+      row = next;
+    }
+    if (p.split == 1) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const int m = mem[slot][c];
+        if (m >= 0) p.effv[(fbase + m) * kFB + f] = make_double2(ar[c], ai[c]);
+      }
+    }
+    __syncwarp();
+  }
+  if (p.split > 1) {  // one window per team
+    __syncthreads();
+    double2* sums = (double2*)had32_dyn;
+    const bool have = g0 + slot / p.split < g1;
+    if (have)
+#pragma unroll
+      for (int c = 0; c < C; ++c) sums[(slot * C + c) * 32 + f] = make_double2(ar[c], ai[c]);
+    __syncthreads();
+    if (!have) return;
+    for (int c = part; c < C; c += p.split) {
+      const int m = mem[slot][c];
+      if (m < 0) continue;
+      double2 s = sums[((slot - part) * C + c) * 32 + f];
+      for (int q = 1; q < p.split; ++q) {
+        const double2 v = sums[((slot - part + q) * C + c) * 32 + f];
+        s.x += v.x;
+        s.y += v.y;
+      }
+      p.effv[(fbase + m) * kFB + f] = s;
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kHad32Threads, 1) hadamard_fp32_kernel(Had32Params p) {
   extern __shared__ __align__(128) unsigned char had32_dyn[];
   __shared__ int win[kHad32Warps][216];
@@ -1563,7 +1602,9 @@ __global__ void __launch_bounds__(kHad32Threads, 1) hadamard_fp32_kernel(Had32Pa
   const int g0 = blockIdx.x * p.groups_per_block;
   const int g1 = min(p.ngroups, g0 + p.groups_per_block);
   const size_t fbase = (size_t)fb * p.nn;
-  if (!had32_load_tile(p.tile, fb, had32_dyn, &bar, p.error, p.wait_limit)) return;
+  if (!had_load_tile<kHad32TileBytes>(p.tile + (size_t)fb * 343 * kFB, had32_dyn, &bar, p.error,
+                                      p.wait_limit))
+    return;
   for (int g = g0 + slot; g < g1; g += kHad32Warps) {
     for (int q = f; q < 216; q += 32) win[slot][q] = p.win[(size_t)g * 216 + q];
     if (f < 8) mem[slot][f] = p.members[(size_t)g * 8 + f];
@@ -1760,7 +1801,9 @@ __global__ void __launch_bounds__(kHadPairThreads, 1) hadamard_fp32_pair_kernel(
   const int g1 = min(p.npairs, g0 + p.pairs_per_block);
   const size_t fbase = (size_t)fb * p.nn;
   const unsigned long long* spec = (const unsigned long long*)p.spec + fbase * kFB + f;
-  if (!had32_load_tile(p.tile, fb, had32_dyn, &bar, p.error, p.wait_limit)) return;
+  if (!had_load_tile<kHad32TileBytes>(p.tile + (size_t)fb * 343 * kFB, had32_dyn, &bar, p.error,
+                                      p.wait_limit))
+    return;
   for (int g = g0 + slot; g < g1; g += kHadPairWarps) {
     for (int q = f; q < 288; q += 32) win[slot][q] = p.win[(size_t)g * 288 + q];
     if (f < 16) mem[slot][f] = p.members[(size_t)g * 16 + f];

@@ -117,7 +117,7 @@ struct kfmm_plan {
   // collects [0] over the kfmm_evaluate_async calls since the last wait
   int* d_error = nullptr;
   long long wait_limit = kMbarSpinLimit;  // tries of the V-list tile-copy wait
-  int had32_groups_per_block = 0;
+  int single_per_block = 0, single_split = 1;  // Hadamard launch shapes (set_had_blocks)
   int p2p_grid = 0;            // resident P2P blocks on the device
   bool nf_minb5 = false;       // mixed near field with 5 resident blocks per SM
   kfmm_tuning tune{};          // launch choices asked for at creation (0 = automatic)
@@ -125,15 +125,14 @@ struct kfmm_plan {
   std::vector<GemmBatch> up_gemms, down_gemms;
   int *fft_nodes = nullptr, *ifft_nodes = nullptr;
   int n_fft = 0, n_ifft = 0;
-  int *win = nullptr, *members = nullptr;
   int n_groups = 0;
-  // mixed form: x-neighbour pairs of groups and the groups left single
+  // x-neighbour pairs of sibling groups and the groups left single
   unsigned long long* pair_rows = nullptr;  // per pair window: rows holding an entry
   unsigned long long* single_rows = nullptr;
   int *pair_win = nullptr, *pair_members = nullptr, *single_win = nullptr,
       *single_members = nullptr;
   int n_pairs = 0, n_singles = 0;
-  int pair_per_block = 0;
+  int pair_per_block = 0, pair_split = 1;
   // tensor-core Hadamard (mixed form) on the complete levels it takes: levels,
   // box -> node maps and the MMAs' B operands; the spectra, the error flag and
   // the unit counter are filled in at launch
@@ -273,8 +272,7 @@ void count_launches(kfmm_plan* p) {
   p->stats.tensor_levels = p->n_tc_levels;
   p->stats.host_pairs = p->host_pairs;
   p->stats.launches = reduces + (p->n_s2m > 0) + (int)p->up_gemms.size() + (p->n_fft > 0) +
-                      (p->prec == KFMM_MIXED ? (p->n_pairs > 0) + (p->n_singles > 0)
-                                             : (p->n_groups > 0)) +
+                      (p->n_pairs > 0) + (p->n_singles > 0) +
                       (p->n_tc_levels > 0) + (p->n_ifft > 0) + (p->n_s2l > 0) +
                       (int)p->down_gemms.size() + (p->n_nf > 0) +
                       (p->prec == KFMM_MIXED ? 0 : 1);  // the plain form's scatter pass
@@ -565,29 +563,38 @@ kfmm_status build_nf_jobs(kfmm_plan* p) {
   return KFMM_OK;
 }
 
-// Mixed Hadamard launch shape: one CTA per SM over (chunks x frequency
-// blocks).  A chunk holds k windows per warp (every warp the same count, so
-// none idles at the end of its CTA); k minimises the span ceil(CTAs / SMs) x
-// (k + 0.1), the 0.1 standing for a CTA's translation-tile load, unless the
-// tuning fixes k.
+// Hadamard launch shapes: one CTA per SM over (chunks x frequency blocks).  A
+// chunk holds k windows per warp (every warp the same count, so none idles at
+// the end of its CTA); k minimises the span ceil(CTAs / SMs) x (k + tile), tile
+// standing for a CTA's translation-tile load (FP32 0.1, FP64 0.2 windows), unless
+// the tuning fixes k.  The FP64 kernel may also give a window to 2, 4 or 8 warps,
+// one window per team: k = 1 / split.
 void set_had_blocks(kfmm_plan* p) {
   const int nfb = p->Fpad / kFB;
-  auto per_block = [&](int items, int warps) {
-    if (p->tune.had_windows > 0) return warps * std::min(p->tune.had_windows, 8);
-    int pick = warps;
+  const bool mixed = p->prec == KFMM_MIXED;
+  auto shape = [&](int items, int warps, int* per, int* split) {
+    *split = 1;
+    if (p->tune.had_windows > 0 && mixed) {
+      *per = warps * std::min(p->tune.had_windows, 8);
+      return;
+    }
+    *per = warps;
     double best = 1e300;
-    for (int k = 1; k <= 8; ++k) {
-      const long long ctas = (long long)((items + warps * k - 1) / (warps * k)) * nfb;
-      const double span = std::ceil((double)ctas / p->num_sms) * (k + 0.1);
+    auto consider = [&](int windows, int s, double k) {
+      const long long ctas = (long long)((items + windows - 1) / windows) * nfb;
+      const double span = std::ceil((double)ctas / p->num_sms) * (k + (mixed ? 0.1 : 0.2));
       if (span < best) {
         best = span;
-        pick = warps * k;
+        *per = windows;
+        *split = s;
       }
-    }
-    return pick;
+    };
+    for (int k = 1; k <= 8; ++k) consider(warps * k, 1, k);
+    if (!mixed)
+      for (int s = 2; s <= warps; s *= 2) consider(warps / s, s, 1.0 / s);
   };
-  p->had32_groups_per_block = per_block(p->n_singles, kHad32Warps);
-  p->pair_per_block = per_block(p->n_pairs, kHadPairWarps);
+  shape(p->n_singles, mixed ? kHad32Warps : kHad64Warps, &p->single_per_block, &p->single_split);
+  shape(p->n_pairs, mixed ? kHadPairWarps : kHad64Warps, &p->pair_per_block, &p->pair_split);
 }
 
 kfmm_status check_tuning(const kfmm_tuning* t) {
@@ -741,11 +748,13 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
     KF_TRY(upload(p, &d, tr));
     p->d_trans = d;
   } else {
-    std::vector<double2> tr((size_t)343 * p->Fpad, make_double2(0.0, 0.0));
+    // the same layout in FP64, 175,616 bytes a tile (hadamard_fp64_kernel)
+    const int nfb = p->Fpad / kFB;
+    std::vector<double2> tr((size_t)nfb * 343 * kFB, make_double2(0.0, 0.0));
     for (int id = 0; id < 343; ++id)
       for (int f = 0; f < F && !adjacent(id); ++f)
-        tr[(size_t)id * p->Fpad + f] = make_double2(op.ue2dc[2 * ((size_t)id * F + f)],
-                                                    op.ue2dc[2 * ((size_t)id * F + f) + 1]);
+        tr[((size_t)(f / kFB) * 343 + id) * kFB + f % kFB] =
+            make_double2(op.ue2dc[2 * ((size_t)id * F + f)], op.ue2dc[2 * ((size_t)id * F + f) + 1]);
     double2* d = nullptr;
     KF_TRY(upload(p, &d, tr));
     p->d_trans = d;
@@ -1045,7 +1054,7 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
         KF_TRY(dalloc(p, &p->tc_counter, 1));
       }
     }
-    if (p->prec == KFMM_MIXED && p->n_groups) {
+    if (p->n_groups) {
       // pair groups whose parents are x-neighbours (x even, x + 1): their
       // windows share 4 of 6 x-positions and form one 8 x 6 x 6 window
       // per parent depth: parent position -> group
@@ -1109,8 +1118,6 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
       KF_TRY(upload(p, &p->single_win, swin));
       KF_TRY(upload(p, &p->single_members, smem));
     }
-    KF_TRY(upload(p, &p->win, win));
-    KF_TRY(upload(p, &p->members, mem));
     p->stats.spectra_bytes = 16.0 * F * ((double)fn.size() + (double)ifn.size());
   }
 
@@ -1280,6 +1287,10 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
                                (int)kTcSmemBytes));
   KF_CUDA(cudaFuncSetAttribute(hadamard_fp32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kHad32TileBytes));
+  KF_CUDA(cudaFuncSetAttribute(hadamard_fp64_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kHad64TileBytes));
+  KF_CUDA(cudaFuncSetAttribute(hadamard_fp64_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kHad64TileBytes));
   KF_CUDA(cudaFuncSetAttribute(hadamard_fp32_pair_kernel,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kHadPairSmemBytes));
@@ -1596,7 +1607,7 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
         KF_CHECK_LAUNCH("hadamard_fp32_pair_kernel");
       }
       if (p->n_singles) {
-        const int gpb = p->had32_groups_per_block;
+        const int gpb = p->single_per_block;
         Had32Params h{p->nn, p->n_singles, gpb, p->single_win, p->single_members, p->single_rows,
                       (const float2*)p->d_trans, (const float2*)p->spec, (float2*)p->effv,
                       p->d_error, p->wait_limit};
@@ -1616,12 +1627,19 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
         KF_CHECK_LAUNCH("hadamard_tc_kernel");
       }
     } else {
-      HadamardParams h{p->nn, p->n_groups, kHadGroupsPerBlock, p->win, p->members,
-                       (const double2*)p->d_trans, p->Fpad, (const double2*)p->spec,
-                       (double2*)p->effv};
-      dim3 grid((p->n_groups + kHadGroupsPerBlock - 1) / kHadGroupsPerBlock, p->Fpad / kFB);
-      hadamard_kernel<<<grid, kHadThreads, 0, S(stream)>>>(h);
-      KF_CHECK_LAUNCH("hadamard_kernel");
+      auto launch = [&](auto kern, int nwin, int per, int split, const int* win, const int* members,
+                        const unsigned long long* rows) {
+        if (nwin == 0) return;
+        Had64Params h{p->nn, nwin, per, split, win, members, rows, (const double2*)p->d_trans,
+                      (const double2*)p->spec, (double2*)p->effv, p->d_error};
+        dim3 grid((nwin + per - 1) / per, p->Fpad / kFB);
+        kern<<<grid, kHad64Threads, kHad64TileBytes, S(stream)>>>(h);
+      };
+      launch(hadamard_fp64_kernel<2>, p->n_pairs, p->pair_per_block, p->pair_split, p->pair_win,
+             p->pair_members, p->pair_rows);
+      launch(hadamard_fp64_kernel<1>, p->n_singles, p->single_per_block, p->single_split,
+             p->single_win, p->single_members, p->single_rows);
+      KF_CHECK_LAUNCH("hadamard_fp64_kernel");
     }
   }
   mark(p, 4, S(stream));
