@@ -826,8 +826,6 @@ p2p_fused_kernel(const P2PMixedParams* params, const P2PJob* jobs, int njobs, in
 struct GemmArgs {
   const double* A;
   int M, K;
-  int ksplit;        // K range per blockIdx.z (multiple of kGemmBK)
-  double* partial;   // split-K: partial sums [z][ncol][M] (no alpha), else NULL
   const double* B;
   const int* boff;
   double* C;
@@ -884,8 +882,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_fp64_dmma_kernel(GemmArg
   const int wm = warp >> 1, wn = warp & 1;
   const int m0 = blockIdx.x * mrows, n0 = blockIdx.y * kGemmBN;
   const int mend = min(g.M, m0 + mrows);
-  const int kb = blockIdx.z * g.ksplit, ke = min(g.K, kb + g.ksplit);
-  const int nslices = ke > kb ? (ke - kb + kGemmBK - 1) / kGemmBK : 0;
+  const int nslices = (g.K + kGemmBK - 1) / kGemmBK;
   if (tid < kGemmBN) {
     const bool in = n0 + tid < g.ncol;
     boff_s[tid] = in ? g.boff[n0 + tid] : -1;
@@ -903,13 +900,13 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_fp64_dmma_kernel(GemmArg
   auto issue = [&](int s) {
     double* As = gsm + (s % kGemmStages) * kGemmStageDoubles;
     double* Bs = As + kGemmBK * kGemmAStride;
-    const int k0 = kb + s * kGemmBK;
+    const int k0 = s * kGemmBK;
 #pragma unroll
     for (int r = 0; r < kGemmRows * kGemmBK / 2 / kGemmThreads; ++r) {
       const int q = tid + r * kGemmThreads;
       const int k = q / (kGemmRows / 2), m = 2 * (q % (kGemmRows / 2));
       const int gm = m0 + m, gk = k0 + k;
-      const bool ok = gm < mend && gk < ke;
+      const bool ok = gm < mend && gk < g.K;
       cp_async16(As + k * kGemmAStride + m, ok ? g.A + (size_t)gk * g.M + gm : g.A, ok);
     }
 #pragma unroll
@@ -917,7 +914,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_fp64_dmma_kernel(GemmArg
       const int q = tid + r * kGemmThreads;
       const int n = q / (kGemmBK / 2), k = 2 * (q % (kGemmBK / 2));
       const int gk = k0 + k, bo = boff_s[n];
-      const bool ok = bo >= 0 && gk < ke;
+      const bool ok = bo >= 0 && gk < g.K;
       cp_async16(Bs + n * kGemmBStride + k, ok ? g.B + (size_t)bo + gk : g.B, ok);
     }
   };
@@ -959,12 +956,8 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_fp64_dmma_kernel(GemmArg
           const int m = m0 + wm * 40 + mi * 8 + (lane >> 2);
           const int n = n0 + wn * 32 + ni * 8 + (lane & 3) * 2 + h;
           if (m < mend && n < g.ncol) {
-            if (g.partial) {
-              g.partial[((size_t)blockIdx.z * g.ncol + n) * g.M + m] = acc[mi][ni][h];
-            } else {
-              const double a = g.alpha ? g.alpha[n] : g.alpha_const;
-              g.C[(size_t)g.coff[n] + m] = a * acc[mi][ni][h];
-            }
+            const double a = g.alpha ? g.alpha[n] : g.alpha_const;
+            g.C[(size_t)g.coff[n] + m] = a * acc[mi][ni][h];
           }
         }
   } else {
@@ -982,8 +975,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_fp64_dmma_kernel(GemmArg
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int nl = wn * 32 + ni * 8 + (lane & 3) * 2 + h;
-          old[ni][h] = !g.partial && m < mend && n0 + nl < g.ncol ? g.C[(size_t)coff_s[nl] + m]
-                                                                  : 0.0;
+          old[ni][h] = m < mend && n0 + nl < g.ncol ? g.C[(size_t)coff_s[nl] + m] : 0.0;
         }
 #pragma unroll
       for (int ni = 0; ni < 4; ++ni)
@@ -991,35 +983,102 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_fp64_dmma_kernel(GemmArg
         for (int h = 0; h < 2; ++h) {
           const int nl = wn * 32 + ni * 8 + (lane & 3) * 2 + h, n = n0 + nl;
           if (m < mend && n < g.ncol) {
-            if (g.partial) {
-              g.partial[((size_t)blockIdx.z * g.ncol + n) * g.M + m] = acc[mi][ni][h];
-            } else {
-              const double v = alpha_s[nl] * acc[mi][ni][h];
-              g.C[(size_t)coff_s[nl] + m] = old[ni][h] + v;
-            }
+            const double v = alpha_s[nl] * acc[mi][ni][h];
+            g.C[(size_t)coff_s[nl] + m] = old[ni][h] + v;
           }
         }
     }
   }
 }
 
-// Split-K: sum the partial products in split order (deterministic), then
-// scale and store as the single-pass kernel would.  A grid-wide pass: the
-// sums of every output tile proceed in parallel (a reduction by each tile's
-// last-arriving block instead serialises 8 x 160 x 64 loads per tile at the
-// end of the launch, measured 0.3 ms slower per solve at 4M points, NP=6).
-__global__ void gemm_splitk_reduce_kernel(GemmArgs g, int nsplit) {
-  const size_t total = (size_t)g.ncol * g.M;
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < total;
-       q += (size_t)gridDim.x * blockDim.x) {
-    const int n = (int)(q / g.M), m = (int)(q % g.M);
-    double sum = 0.0;
-    for (int z = 0; z < nsplit; ++z) sum += g.partial[((size_t)z * g.ncol + n) * g.M + m];
+// The same product in small tiles, operands straight from global memory (L2)
+// into the fragments: a CTA computes 40 rows x 16 wn columns, its 8 warps being wn
+// column groups times wk = 8 / wn shares of K, whose sums meet in shared memory.
+// No pipeline to fill, no split-K pass: what bounds a level product of a few
+// hundred columns is the latency of its start and of the passes after it.
+constexpr int kSmallRows = 40, kSmallCols = 16, kSmallWarps = 8;
+constexpr int kSmallOut = kSmallRows * kSmallCols;  // outputs of one warp tile
+
+__global__ void __launch_bounds__(32 * kSmallWarps, 2) gemm_fp64_small_kernel(GemmArgs g, int wn) {
+  __shared__ double red[kSmallWarps][kSmallOut];  // [warp][col][row]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wk = kSmallWarps / wn, cg = warp % wn, ks = warp / wn;
+  const int m0 = blockIdx.x * kSmallRows, n0 = blockIdx.y * (kSmallCols * wn);
+  const int r = lane >> 2, c = lane & 3;
+  // this warp's K range, a multiple of 4 but for the end
+  const int quads = (g.K + 3) / 4;
+  const int k0 = 4 * (quads * ks / wk), k1 = min(g.K, 4 * (quads * (ks + 1) / wk));
+  const double* ap[5];
+#pragma unroll
+  for (int i = 0; i < 5; ++i)  // rows beyond the matrix repeat its last (not stored)
+    ap[i] = g.A + (size_t)(k0 + c) * g.M + min(g.M - 1, m0 + 8 * i + r);
+  const double* bp[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    bp[j] = g.B + g.boff[min(g.ncol - 1, n0 + cg * kSmallCols + 8 * j + r)] + k0 + c;
+  double acc[5][2][2];
+#pragma unroll
+  for (int i = 0; i < 5; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  int k = k0;
+  constexpr int U = 4;
+  for (; k + 4 * U <= k1; k += 4 * U) {
+    double af[U][5], bf[U][2];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+      for (int i = 0; i < 5; ++i) af[u][i] = __ldg(ap[i] + (size_t)(4 * u) * g.M);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) bf[u][j] = bp[j][4 * u];
+    }
+#pragma unroll
+    for (int i = 0; i < 5; ++i) ap[i] += (size_t)(4 * U) * g.M;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) bp[j] += 4 * U;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int i = 0; i < 5; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) dmma_884(acc[i][j][0], acc[i][j][1], af[u][i], bf[u][j]);
+  }
+  if (k < k1) {  // up to 15 more, zero beyond the range
+    double af[U][5], bf[U][2];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = k + 4 * u + c < k1;
+#pragma unroll
+      for (int i = 0; i < 5; ++i) af[u][i] = in ? __ldg(ap[i] + (size_t)(4 * u) * g.M) : 0.0;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) bf[u][j] = in ? bp[j][4 * u] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int i = 0; i < 5; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) dmma_884(acc[i][j][0], acc[i][j][1], af[u][i], bf[u][j]);
+  }
+#pragma unroll
+  for (int i = 0; i < 5; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        red[warp][(8 * j + 2 * c + h) * kSmallRows + 8 * i + r] = acc[i][j][h];
+  __syncthreads();
+  // outputs: 40 consecutive rows of a column by consecutive threads
+  for (int q = threadIdx.x; q < wn * kSmallOut; q += 32 * kSmallWarps) {
+    const int w = q / kSmallOut, e = q % kSmallOut;
+    const int m = m0 + e % kSmallRows, n = n0 + w * kSmallCols + e / kSmallRows;
+    if (m >= g.M || n >= g.ncol) continue;
+    double s = red[w][e];
+    for (int z = 1; z < wk; ++z) s += red[w + z * wn][e];
     const double a = g.alpha ? g.alpha[n] : g.alpha_const;
-    double* c = g.C + (size_t)g.coff[n] + m;
-    const double v = a * sum;
-    if (g.accumulate) *c += v;
-    else *c = v;
+    double* o = g.C + (size_t)g.coff[n] + m;
+    if (g.accumulate) *o += a * s;
+    else *o = a * s;
   }
 }
 

@@ -53,7 +53,8 @@ void set_error(const std::string& msg) { g_error = msg; }
 struct GemmBatch {
   const double* A;
   int M, K;
-  int chunks, mrows, nsplit, ksplit;  // launch shape, fixed at plan time
+  int chunks, mrows;  // launch shape in large tiles
+  int wn;             // small tiles: column groups per CTA; 0: large tiles
   const double* B;
   int* boff;  // device
   double* C;
@@ -153,8 +154,6 @@ struct kfmm_plan {
   double host_pairs = 0.0;
   kfmm_stats stats{};
   int num_sms = 148;
-  double* splitk = nullptr;   // split-K partial sums, shared by the level GEMMs
-  size_t splitk_doubles = 0;
   bool timing = false;
   // timing marks (kfmm_enable_timing): 0 start, 1 S2M pairs done, 2 up done,
   // 3 forward FFT, 4 Hadamard, 5 inverse FFT (V done), 6 S2L (X done),
@@ -212,66 +211,26 @@ kfmm_status upload(kfmm_plan* p, T** ptr, const std::vector<T>& h) {
     if (s_ != KFMM_OK) return s_;  \
   } while (0)
 
-// Split K when the launch would give fewer than two blocks per SM.  The split
-// count minimises (waves of blocks) x (16-deep K slices per block) plus the
-// split-K partial sums' traffic, 16 B per entry per split, counted at ~12.5 MB
-// per slice-wave (the kernel's measured rate): one wave of half-K blocks
-// beats two waves of third-K blocks.  Up to max(8, K / 64) ways unless the
-// plan's tuning says otherwise (measured on 4M points: allowing 8 ways to the
-// short-K products, K = P or Q, took 0.25 ms off the ellipsoid-surface solve
-// at NP=4 and 0.05 ms off the uniform one at NP=6, against K / 64 ways).
-constexpr int kSplitKAuto = 8;
-void choose_split(const kfmm_plan* p, GemmBatch& g) {
-  const int M = g.M, K = g.K;
-  const int blocks = g.chunks * ((g.ncol + kGemmBN - 1) / kGemmBN);
+// Large tiles (160 x 64, kGemmRows x kGemmBN) when they give every SM its two
+// blocks; else small tiles, with the fewest column groups per CTA (the most
+// shares of K, up to the tuning's splitk_max) that leave at most two CTAs per SM.
+void choose_tiles(const kfmm_plan* p, GemmBatch& g) {
   const int want = 2 * p->num_sms;
-  g.nsplit = 1;
-  g.ksplit = (K + kGemmBK - 1) / kGemmBK * kGemmBK;
-  if (blocks >= want) return;
-  double best = 1e300;
-  const int smax = p->tune.splitk_max > 0 ? p->tune.splitk_max : std::max(kSplitKAuto, K / 64);
-  for (int s = 1; s <= smax; ++s) {
-    const int ks = ((K + s - 1) / s + kGemmBK - 1) / kGemmBK * kGemmBK;
-    const int ns = (K + ks - 1) / ks;
-    const double waves = std::ceil((double)blocks * ns / want);
-    const double traffic = ns > 1 ? ns * 16.0 * M * (double)g.ncol / 12.5e6 : 0.0;
-    const double cost = waves * (ks / kGemmBK) + traffic;
-    if (cost < best) {
-      best = cost;
-      g.nsplit = ns;
-      g.ksplit = ks;
-    }
-  }
-}
-
-// Split-K scratch the plan's level products need (doubles).
-size_t splitk_need(const kfmm_plan* p) {
-  size_t n = 0;
-  for (const auto* v : {&p->up_gemms, &p->down_gemms})
-    for (const GemmBatch& g : *v)
-      if (g.nsplit > 1) n = std::max(n, (size_t)g.nsplit * g.ncol * g.M);
-  return n;
-}
-
-// Split-K partial-sum buffer at least as large as the level products need.
-kfmm_status ensure_splitk(kfmm_plan* p) {
-  const size_t need = splitk_need(p);
-  if (need > p->splitk_doubles) {
-    dfree(p, p->splitk);
-    KF_TRY(dalloc(p, &p->splitk, need));
-    p->splitk_doubles = need;
-  }
-  return KFMM_OK;
+  g.wn = 0;
+  if (g.chunks * ((g.ncol + kGemmBN - 1) / kGemmBN) >= want) return;
+  const int mt = (g.M + kSmallRows - 1) / kSmallRows;
+  auto ctas = [&](int wn) { return mt * ((g.ncol + kSmallCols * wn - 1) / (kSmallCols * wn)); };
+  g.wn = 1;
+  if (p->tune.splitk_max > 0)
+    while (kSmallWarps / g.wn > p->tune.splitk_max) g.wn *= 2;
+  while (g.wn < kSmallWarps && ctas(g.wn) > want) g.wn *= 2;
 }
 
 // Kernel launches of one kfmm_run (kfmm_plan_stats.launches).
 void count_launches(kfmm_plan* p) {
-  int reduces = 0;
-  for (const auto* v : {&p->up_gemms, &p->down_gemms})
-    for (const GemmBatch& g : *v) reduces += g.nsplit > 1;
   p->stats.tensor_levels = p->n_tc_levels;
   p->stats.host_pairs = p->host_pairs;
-  p->stats.launches = reduces + (p->n_s2m > 0) + (int)p->up_gemms.size() + (p->n_fft > 0) +
+  p->stats.launches = (p->n_s2m > 0) + (int)p->up_gemms.size() + (p->n_fft > 0) +
                       (p->n_pairs > 0) + (p->n_singles > 0) +
                       (p->n_tc_levels > 0) + (p->n_ifft > 0) + (p->n_s2l > 0) +
                       (int)p->down_gemms.size() + (p->n_nf > 0) +
@@ -304,7 +263,7 @@ kfmm_status add_gemm(kfmm_plan* p, std::vector<GemmBatch>& out, const double* A,
   if (alpha) KF_TRY(upload(p, &g.alpha, *alpha));
   g.chunks = (M + kGemmRows - 1) / kGemmRows;
   g.mrows = ((M + g.chunks - 1) / g.chunks + 7) / 8 * 8;
-  choose_split(p, g);
+  choose_tiles(p, g);
   p->stats.gemm_flops += 2.0 * M * (double)K * g.ncol;
   out.push_back(g);
   return KFMM_OK;
@@ -312,20 +271,20 @@ kfmm_status add_gemm(kfmm_plan* p, std::vector<GemmBatch>& out, const double* A,
 
 kfmm_status launch_gemms(const kfmm_plan* p, const std::vector<GemmBatch>& gs, cudaStream_t st) {
   for (const GemmBatch& b : gs) {
-    GemmArgs a{b.A, b.M, b.K, b.ksplit, b.nsplit > 1 ? p->splitk : nullptr, b.B, b.boff, b.C,
-               b.coff, b.alpha, b.alpha_const, b.ncol, b.accumulate};
-    dim3 grid(b.chunks, (b.ncol + kGemmBN - 1) / kGemmBN, b.nsplit);
+    GemmArgs a{b.A, b.M, b.K, b.B, b.boff, b.C, b.coff, b.alpha, b.alpha_const, b.ncol, b.accumulate};
+    if (b.wn) {
+      const int cols = kSmallCols * b.wn;
+      dim3 grid((b.M + kSmallRows - 1) / kSmallRows, (b.ncol + cols - 1) / cols);
+      gemm_fp64_small_kernel<<<grid, 32 * kSmallWarps, 0, st>>>(a, b.wn);
+      KF_CHECK_LAUNCH("gemm_fp64_small_kernel");
+      continue;
+    }
+    dim3 grid(b.chunks, (b.ncol + kGemmBN - 1) / kGemmBN);
     if (b.accumulate)
       gemm_fp64_dmma_kernel<true><<<grid, kGemmThreads, kGemmSmemBytes, st>>>(a, b.mrows);
     else
       gemm_fp64_dmma_kernel<false><<<grid, kGemmThreads, kGemmSmemBytes, st>>>(a, b.mrows);
     KF_CHECK_LAUNCH("gemm_fp64_dmma_kernel");
-    if (b.nsplit > 1) {
-      const size_t total = (size_t)b.ncol * b.M;
-      const int blocks = (int)std::min<size_t>((total + 255) / 256, 4 * (size_t)p->num_sms);
-      gemm_splitk_reduce_kernel<<<blocks, 256, 0, st>>>(a, b.nsplit);
-      KF_CHECK_LAUNCH("gemm_splitk_reduce_kernel");
-    }
   }
   return KFMM_OK;
 }
@@ -1296,7 +1255,6 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
                                (int)kHadPairSmemBytes));
   set_had_blocks(p);
 
-  KF_TRY(ensure_splitk(p));
   KF_TRY(dalloc(p, &p->job_counter, 3));
   KF_TRY(dalloc(p, &p->d_error, 2));
   KF_CUDA(cudaMemset(p->d_error, 0, 2 * sizeof(int)));
@@ -1502,9 +1460,8 @@ kfmm_status kfmm_plan_set_tuning(kfmm_plan* p, const kfmm_tuning* tuning) {
   set_had_blocks(p);
   if (p->tune.splitk_max != old.splitk_max) {
     for (auto* v : {&p->up_gemms, &p->down_gemms})
-      for (GemmBatch& g : *v) choose_split(p, g);
-    KF_TRY(ensure_splitk(p));
-    count_launches(p);
+      for (GemmBatch& g : *v) choose_tiles(p, g);
+      count_launches(p);
   }
   return KFMM_OK;
 }
