@@ -60,6 +60,9 @@ struct P2PParams {
   const double* sp_de;
   const double* sp_dc;
   double* out;
+  // near field: target i of a job goes to out[out_perm[J.out + i]], the original
+  // order (no scatter pass afterwards); null: out[J.out + i]
+  const int* out_perm;
   int P, Q;
 };
 
@@ -79,9 +82,6 @@ struct P2PMixedParams {
   const int* entry_ids;
   const int* src_beg;
   const int* src_num;
-  // near field: target i of a job goes to out[out_perm[J.out + i]], the
-  // original order (no scatter pass afterwards); null: out[J.out + i]
-  const int* out_perm;
 };
 template <bool kMixed>
 using P2PArgs = typename std::conditional<kMixed, P2PMixedParams, P2PParams>::type;
@@ -437,7 +437,7 @@ __device__ __forceinline__ void row_job_mixed(const P2PMixedParams& a, const P2P
     const int i = lane + 32 * t;
     if (i < J.tcnt) {
       const double r = kOOFP * acc[t];
-      double* o = p.out + (a.out_perm ? a.out_perm[J.out + i] : J.out + i);
+      double* o = p.out + (p.out_perm ? p.out_perm[J.out + i] : J.out + i);
       if (J.mode) *o += r;
       else *o = r;
     }
@@ -653,7 +653,7 @@ __device__ __forceinline__ void team_job_mixed(const P2PMixedParams& a, const P2
     }
     __syncwarp();
   }
-  store_job<NS, G, true>(J, p.out, a.out_perm, acc, lane, red);
+  store_job<NS, G, true>(J, p.out, p.out_perm, acc, lane, red);
 }
 
 // Plain FP64 form: the same walk, sources staged as double4.
@@ -691,7 +691,7 @@ __device__ __forceinline__ void warp_job_fp64(const P2PParams& p, const P2PJob& 
     else pairs_fp64<NS, false, G>(tx, ty, tz, acc, mine, (cnt + G - 1) / G);
     __syncwarp();
   }
-  store_job<NS, G, kIsTeam>(J, p.out, nullptr, acc, lane, red);
+  store_job<NS, G, kIsTeam>(J, p.out, p.out_perm, acc, lane, red);
 }
 
 // Shared memory of one P2P warp: its chunk of 32 sources and its staged entries.
@@ -1953,8 +1953,8 @@ __global__ void __launch_bounds__(kHadPairThreads, 1) hadamard_fp32_pair_kernel(
 #include "hadamard_tc.cuh"
 
 // ---------------------------------------------------------------------------
-// Point reordering (fmm/evaluate.cc:14-52 on the host in the reference) and
-// the final scatter to original order (copy_trg_val, fmm/cuda.cu:2543-2565).
+// Point reordering (fmm/evaluate.cc:14-52 on the host in the reference); the near
+// field stores original order itself (copy_trg_val, fmm/cuda.cu:2543-2565).
 // ---------------------------------------------------------------------------
 // Points to leaf order, driven from the original order: point k (read
 // coalesced) goes to leaf-order position inv[k], one full 32-byte record
@@ -1983,12 +1983,6 @@ __global__ void gather_pot_kernel(int n, const int* perm, const double* pot_orig
                                   double* pot_leaf) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     pot_leaf[i] = pot_orig[perm[i]];
-}
-
-__global__ void scatter_pot_kernel(int n, const int* perm, const double* pot_leaf,
-                                   double* pot_orig) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    pot_orig[perm[i]] = pot_leaf[i];
 }
 
 // error[1] |= error[0]: the per-solve flag of a bounded wait folded into the

@@ -233,8 +233,7 @@ void count_launches(kfmm_plan* p) {
   p->stats.launches = (p->n_s2m > 0) + (int)p->up_gemms.size() + (p->n_fft > 0) +
                       (p->n_pairs > 0) + (p->n_singles > 0) +
                       (p->n_tc_levels > 0) + (p->n_ifft > 0) + (p->n_s2l > 0) +
-                      (int)p->down_gemms.size() + (p->n_nf > 0) +
-                      (p->prec == KFMM_MIXED ? 0 : 1);  // the plain form's scatter pass
+                      (int)p->down_gemms.size() + (p->n_nf > 0);
 }
 
 kfmm_status add_gemm(kfmm_plan* p, std::vector<GemmBatch>& out, const double* A, int M, int K,
@@ -289,7 +288,8 @@ kfmm_status launch_gemms(const kfmm_plan* p, const std::vector<GemmBatch>& gs, c
   return KFMM_OK;
 }
 
-P2PParams p2p_params(const kfmm_plan* p, const P2PJob* jobs, const P2PEntry* ent, double* out) {
+P2PParams p2p_params(const kfmm_plan* p, const P2PJob* jobs, const P2PEntry* ent, double* out,
+                     const int* out_perm = nullptr) {
   P2PParams q;
   q.jobs = jobs;
   q.entries = ent;
@@ -303,31 +303,28 @@ P2PParams p2p_params(const kfmm_plan* p, const P2PJob* jobs, const P2PEntry* ent
   q.sp_de = p->d_sp_de;
   q.sp_dc = p->d_sp_dc;
   q.out = out;
+  q.out_perm = out_perm;
   q.P = p->P;
   q.Q = p->Q;
   return q;
 }
 
-P2PMixedParams p2p_mixed_params(const kfmm_plan* p, const P2PParams& q, const int* ids,
-                                const int* out_perm = nullptr) {
+P2PMixedParams p2p_mixed_params(const kfmm_plan* p, const P2PParams& q, const int* ids) {
   P2PMixedParams m;
   m.p = q;
   m.src4f = p->src4f;
   m.ctrf = p->ctrf;
   m.spf_ue = p->d_spf_ue;
   m.spf_de = p->d_spf_de;
-  m.out_perm = out_perm;
   m.entry_ids = ids;
   m.src_beg = p->d_src_beg;
   m.src_num = p->d_src_num;
   return m;
 }
 
-// The near field's output: the mixed form writes the potentials in original
-// order directly (its kernel takes the target permutation), the plain form
-// in leaf order for the scatter pass.
-double* near_field_out(const kfmm_plan* p) {
-  return p->prec == KFMM_MIXED ? p->pot_orig : p->pot_leaf;
+// The near field's arguments: it writes the potentials in original order itself.
+P2PParams near_field_params(const kfmm_plan* p) {
+  return p2p_params(p, p->nf_jobs, p->nf_ent, p->pot_orig, p->d_trg_perm);
 }
 
 FFTParams fft_params(const kfmm_plan* p) {
@@ -1338,10 +1335,9 @@ kfmm_status launch_fft(int np, bool mixed, bool forward, int nboxes, int num_sms
 kfmm_status launch_p2p(const kfmm_plan* p, int which, int njobs, const P2PParams& q,
                        const int* ids, void* stream, const char* what) {
   const bool mixed = p->prec == KFMM_MIXED;
-  const int* perm = which == 2 ? p->d_trg_perm : nullptr;
   if (which == 2 && p->nf_team) {
     if (mixed)
-      p2p_team_kernel<true><<<njobs, 32 * kTeam, 0, S(stream)>>>(p2p_mixed_params(p, q, ids, perm));
+      p2p_team_kernel<true><<<njobs, 32 * kTeam, 0, S(stream)>>>(p2p_mixed_params(p, q, ids));
     else
       p2p_team_kernel<false><<<njobs, 32 * kTeam, 0, S(stream)>>>(q);
   } else {
@@ -1354,10 +1350,10 @@ kfmm_status launch_p2p(const kfmm_plan* p, int which, int njobs, const P2PParams
       p2p_warp_kernel<false><<<blocks, 32 * kWarpJobsPerBlock, 0, S(stream)>>>(q, njobs, counter);
     else if (five)
       p2p_warp_kernel<true, 5><<<blocks, 32 * kWarpJobsPerBlock, 0, S(stream)>>>(
-          p2p_mixed_params(p, q, ids, perm), njobs, counter);
+          p2p_mixed_params(p, q, ids), njobs, counter);
     else
       p2p_warp_kernel<true><<<blocks, 32 * kWarpJobsPerBlock, 0, S(stream)>>>(
-          p2p_mixed_params(p, q, ids, perm), njobs, counter);
+          p2p_mixed_params(p, q, ids), njobs, counter);
   }
   KF_CHECK_LAUNCH(std::string("p2p kernel (") + what + ")");
   return KFMM_OK;
@@ -1630,8 +1626,7 @@ kfmm_status near_field(kfmm_plan* p, void* stream) {
     return KFMM_ERR_STATE;
   }
   if (p->n_nf) {
-    KF_TRY(launch_p2p(p, 2, p->n_nf, p2p_params(p, p->nf_jobs, p->nf_ent, near_field_out(p)),
-                      p->nf_ids, stream, "near field"));
+    KF_TRY(launch_p2p(p, 2, p->n_nf, near_field_params(p), p->nf_ids, stream, "near field"));
   }
   return KFMM_OK;
 }
@@ -1656,11 +1651,6 @@ kfmm_status kfmm_ulist_calc(kfmm_plan* p, void* stream) {
 
 kfmm_status kfmm_copy_trg_val(kfmm_plan* p, double* pot_host, void* stream) {
   if (!p) return KFMM_ERR_INVALID;
-  if (p->prec != KFMM_MIXED) {  // the mixed near field wrote pot_orig itself
-    scatter_pot_kernel<<<592, 256, 0, S(stream)>>>(p->nt, p->d_trg_perm, p->pot_leaf,
-                                                   p->pot_orig);
-    KF_CHECK_LAUNCH("scatter_pot_kernel");
-  }
   if (pot_host) {
     KF_CUDA(cudaMemcpyAsync(pot_host, p->pot_orig, sizeof(double) * p->nt, cudaMemcpyDeviceToHost,
                             S(stream)));
@@ -1922,7 +1912,7 @@ kfmm_status kfmm_read_array(kfmm_plan* p, int which, double* out, size_t count) 
     return KFMM_ERR_INVALID;
   }
   KF_CUDA(cudaDeviceSynchronize());
-  if (which == 3 && p->prec == KFMM_MIXED) {  // leaf-order view of pot_orig
+  if (which == 3) {  // leaf-order view of pot_orig
     gather_pot_kernel<<<592, 256>>>(p->nt, p->d_trg_perm, p->pot_orig, p->pot_leaf);
     KF_CHECK_LAUNCH("gather_pot_kernel");
     KF_CUDA(cudaDeviceSynchronize());
@@ -2032,8 +2022,8 @@ kfmm_status kfmm_batch_create(kfmm_plan* const* plans, int nplans, int nstreams,
     std::vector<P2PMixedParams> mparams(mixed ? nplans : 0);
     for (int i = 0; i < nplans; ++i) {
       kfmm_plan* p = plans[i];
-      params[i] = p2p_params(p, p->nf_jobs, p->nf_ent, near_field_out(p));
-      if (mixed) mparams[i] = p2p_mixed_params(p, params[i], p->nf_ids, p->d_trg_perm);
+      params[i] = near_field_params(p);
+      if (mixed) mparams[i] = p2p_mixed_params(p, params[i], p->nf_ids);
     }
     const size_t pbytes = mixed ? sizeof(P2PMixedParams) * nplans : sizeof(P2PParams) * nplans;
     const void* psrc = mixed ? (const void*)mparams.data() : (const void*)params.data();
@@ -2088,10 +2078,6 @@ kfmm_status kfmm_batch_create(kfmm_plan* const* plans, int nplans, int nstreams,
       set_error("kfmm_batch_create: fused near-field launch failed");
       st = KFMM_ERR_CUDA;
     }
-    fork();
-    for (int i = 0; i < nplans && st == KFMM_OK; ++i)
-      st = kfmm_copy_trg_val(plans[i], nullptr, b->streams[i % nstreams]);
-    join();
   }
   e = cudaStreamEndCapture(origin, &b->graph);
   if (st != KFMM_OK) {
