@@ -1408,7 +1408,38 @@ __global__ void __launch_bounds__(kFFTThreads) ifft_trg_np_kernel(FFTParams p) {
 // x meet, for each of the 4 (cy, cz) member pairs, one row of 7 translation
 // spectra.  Pairs of sibling groups whose parents are x-neighbours (parent x even
 // and x + 1) share one 8 x 6 x 6 window, so each translation value serves both.
-constexpr int kHadMaxWin = 288;  // 8 x 6 x 6
+// One launch takes the windows of both kinds (blocks [0, pairs.chunks) the pairs').
+struct HadSet {
+  int nwin = 0, win_per_block = 1, chunks = 0;
+  int split = 1;  // warps that share a window (then one window per team of warps)
+  const int* win = nullptr;      // nwin x (4 + 2H) x 6 x 6 node ids, x fastest (-1 = absent)
+  const int* members = nullptr;  // nwin x 8H node ids (-1 = no V list)
+  // per window: bit wy + 6 wz set if the row has an entry
+  const unsigned long long* rows = nullptr;
+};
+
+// Groups whose windows are mostly empty (clouds on surfaces): their present
+// entries one by one.  Entry (node, k): the source spectrum of `node` meets
+// translation spectrum k - 49 cz - 7 cy - cx for member (cx, cy, cz), so an entry
+// costs 8 translation loads and 8 multiply-adds whatever its place, where a row of
+// a dense window costs 28 loads and 48 a group.
+struct HadSparse {
+  int n = 0, per_block = 1, chunks = 0;
+  const int* ptr = nullptr;      // n + 1
+  const int2* ent = nullptr;
+  const int* members = nullptr;  // n x 8
+};
+__device__ __forceinline__ constexpr int had_member_offset(int c) {
+  return 49 * (c & 1) + 7 * ((c >> 1) & 1) + (c >> 2);
+}
+
+// The rows of a window that warp `part` of `split` takes.
+__device__ __forceinline__ unsigned long long had_rows_of(int part, int split) {
+  if (split == 1) return ~0ull;
+  unsigned long long m = 0ull;
+  for (int r = part; r < 36; r += split) m |= 1ull << r;
+  return m;
+}
 
 // A row of the translation table at (dy, dz) with |dy| <= 1 and |dz| <= 1:
 // its entries dx = -1, 0, 1 (k = 2, 3, 4 of the row) are adjacent offsets,
@@ -1514,22 +1545,23 @@ __device__ __forceinline__ bool had_load_tile(const void* tile, unsigned char* d
 // Plain FP64 form, one CTA per SM: the frequency block's 343 translation spectra
 // (175,616 B) are brought into shared memory by bulk asynchronous copies, a warp
 // takes one window of H sibling groups (H = 2: an x-pair), all 8 H members'
-// sums in registers.  Bound by the FP64 pipe: a row of H = 2 is 384 multiply-adds
-// a lane (192 cycles of the SM's pipe) against 112 shared-memory wavefronts of
-// translation values and 32 of sources; with one group a window the wavefronts
-// outweighed the multiply-adds.
+// sums in registers.  Bound by the FP64 pipe and the latency of its operations: a
+// row of H = 2 is 384 multiply-adds a lane (192 cycles of the SM's pipe) against
+// 112 shared-memory wavefronts of translation values and 32 of sources; with one
+// group a window the wavefronts outweighed the multiply-adds.  4M uniform points,
+// NP 6: 3.98 ms one group a window through L1, 2.96 ms with 8 warps (pipe 42%
+// busy, fixed-latency waits the first stall), 2.63 ms with 12 (168 registers).
 // Where there are fewer windows than warps on the device, `split` warps share a
 // window, each taking every split-th of its rows; their sums meet in shared
 // memory (over the tile, once every warp is done with it) and are added in order.
-constexpr int kHad64Threads = 256;
+constexpr int kHad64Threads = 384;
 constexpr int kHad64Warps = kHad64Threads / 32;
 constexpr unsigned kHad64TileBytes = 343u * kFB * 16u;  // 175,616
 
 struct Had64Params {
-  int nn, nwin, win_per_block, split;
-  const int* win;      // nwin x (4 + 2H) x 6 x 6 node ids, x fastest (-1 = absent)
-  const int* members;  // nwin x 8H node ids (-1 = no V list)
-  const unsigned long long* rows;  // per window: bit wy + 6 wz set if the row has an entry
+  int nn;
+  HadSet pairs, singles;
+  HadSparse sparse;
   const double2* tile;  // [fb][343][32], zero for |delta|_inf <= 1 and f >= F
   const double2* spec;
   double2* effv;
@@ -1537,35 +1569,25 @@ struct Had64Params {
 };
 
 template <int H>
-__global__ void __launch_bounds__(kHad64Threads, 1) hadamard_fp64_kernel(Had64Params p) {
+__device__ __forceinline__ void had64_windows(const Had64Params& p, const HadSet& q, int chunk,
+                                              int (*win)[288], int (*mem)[16],
+                                              unsigned char* had32_dyn) {
   constexpr int WX = 4 + 2 * H, C = 8 * H;
-  extern __shared__ __align__(128) unsigned char had32_dyn[];
-  __shared__ int win[kHad64Warps][36 * WX];
-  __shared__ int mem[kHad64Warps][C];
-  __shared__ __align__(8) unsigned long long bar;
   const double2* tsm = (const double2*)had32_dyn;
-  const int fb = blockIdx.y;
   const int f = threadIdx.x & 31, slot = threadIdx.x >> 5;
-  const int teams = kHad64Warps / p.split, part = slot % p.split;
-  const int g0 = blockIdx.x * p.win_per_block;
-  const int g1 = min(p.nwin, g0 + p.win_per_block);
-  const size_t fbase = (size_t)fb * p.nn;
+  const int teams = kHad64Warps / q.split, part = slot % q.split;
+  const int g0 = chunk * q.win_per_block;
+  const int g1 = min(q.nwin, g0 + q.win_per_block);
+  const size_t fbase = (size_t)blockIdx.y * p.nn;
   const double2* spec = p.spec + fbase * kFB + f;
-  if (!had_load_tile<kHad64TileBytes>(p.tile + (size_t)fb * 343 * kFB, had32_dyn, &bar, p.error,
-                                      kMbarSpinLimit))
-    return;
-  unsigned long long mine = ~0ull;  // this warp's rows of a window
-  if (p.split > 1) {
-    mine = 0ull;
-    for (int r = part; r < 36; r += p.split) mine |= 1ull << r;
-  }
+  const unsigned long long mine = had_rows_of(part, q.split);
   double ar[C], ai[C];
-  for (int g = g0 + slot / p.split; g < g1; g += teams) {
-    for (int q = f; q < 36 * WX; q += 32) win[slot][q] = p.win[(size_t)g * (36 * WX) + q];
-    if (f < C) mem[slot][f] = p.members[(size_t)g * C + f];
+  for (int g = g0 + slot / q.split; g < g1; g += teams) {
+    for (int k = f; k < 36 * WX; k += 32) win[slot][k] = q.win[(size_t)g * (36 * WX) + k];
+    if (f < C) mem[slot][f] = q.members[(size_t)g * C + f];
     __syncwarp();
     const int* w = win[slot];
-    unsigned long long rows = p.rows[g] & mine;
+    unsigned long long rows = q.rows[g] & mine;
 #pragma unroll
     for (int c = 0; c < C; ++c) ar[c] = ai[c] = 0.0;
     double2 nxt[WX];
@@ -1618,7 +1640,7 @@ __global__ void __launch_bounds__(kHad64Threads, 1) hadamard_fp64_kernel(Had64Pa
       }
       row = next;
     }
-    if (p.split == 1) {
+    if (q.split == 1) {
 #pragma unroll
       for (int c = 0; c < C; ++c) {
         const int m = mem[slot][c];
@@ -1627,27 +1649,98 @@ __global__ void __launch_bounds__(kHad64Threads, 1) hadamard_fp64_kernel(Had64Pa
     }
     __syncwarp();
   }
-  if (p.split > 1) {  // one window per team
+  if (q.split > 1) {  // one window per team
     __syncthreads();
     double2* sums = (double2*)had32_dyn;
-    const bool have = g0 + slot / p.split < g1;
+    const bool have = g0 + slot / q.split < g1;
     if (have)
 #pragma unroll
       for (int c = 0; c < C; ++c) sums[(slot * C + c) * 32 + f] = make_double2(ar[c], ai[c]);
     __syncthreads();
     if (!have) return;
-    for (int c = part; c < C; c += p.split) {
+    for (int c = part; c < C; c += q.split) {
       const int m = mem[slot][c];
       if (m < 0) continue;
       double2 s = sums[((slot - part) * C + c) * 32 + f];
-      for (int q = 1; q < p.split; ++q) {
-        const double2 v = sums[((slot - part + q) * C + c) * 32 + f];
+      for (int k = 1; k < q.split; ++k) {
+        const double2 v = sums[((slot - part + k) * C + c) * 32 + f];
         s.x += v.x;
         s.y += v.y;
       }
       p.effv[(fbase + m) * kFB + f] = s;
     }
   }
+}
+
+// Sparse groups, one per warp at a time: entries read 32 at once, one per lane, and
+// handed round; the next entries' spectra are loaded while the current ones are
+// multiplied.
+__device__ __forceinline__ void had64_sparse(const Had64Params& p, int chunk,
+                                             const double2* tsm) {
+  const HadSparse& q = p.sparse;
+  const int f = threadIdx.x & 31, slot = threadIdx.x >> 5;
+  const size_t fbase = (size_t)blockIdx.y * p.nn;
+  const double2* spec = p.spec + fbase * kFB + f;
+  const int g1 = min(q.n, (chunk + 1) * q.per_block);
+  for (int g = chunk * q.per_block + slot; g < g1; g += kHad64Warps) {
+    const int end = q.ptr[g + 1];
+    double ar[8], ai[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) ar[c] = ai[c] = 0.0;
+    for (int e0 = q.ptr[g]; e0 < end; e0 += 32) {
+      const int n = min(32, end - e0);
+      const int2 mine = f < n ? q.ent[e0 + f] : make_int2(0, 0);
+      constexpr int U = 4;
+      double2 nxt[U];
+      auto fetch = [&](int i) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int node = __shfl_sync(0xffffffffu, mine.x, i + u);
+          nxt[u] = i + u < n ? spec[(size_t)node * kFB] : make_double2(0.0, 0.0);
+        }
+      };
+      fetch(0);
+      for (int i = 0; i < n; i += U) {
+        double2 v[U];
+        const double2* t[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          v[u] = nxt[u];
+          const int k = __shfl_sync(0xffffffffu, mine.y, i + u);
+          t[u] = tsm + (i + u < n ? k : had_member_offset(7)) * kFB + f;
+        }
+        if (i + U < n) fetch(i + U);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const double2 w = t[u][-had_member_offset(c) * kFB];
+            ar[c] = fma(-w.y, v[u].y, fma(w.x, v[u].x, ar[c]));
+            ai[c] = fma(w.y, v[u].x, fma(w.x, v[u].y, ai[c]));
+          }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int m = q.members[(size_t)g * 8 + c];
+      if (m >= 0) p.effv[(fbase + m) * kFB + f] = make_double2(ar[c], ai[c]);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kHad64Threads, 1) hadamard_fp64_kernel(Had64Params p) {
+  extern __shared__ __align__(128) unsigned char had32_dyn[];
+  __shared__ int win[kHad64Warps][288];
+  __shared__ int mem[kHad64Warps][16];
+  __shared__ __align__(8) unsigned long long bar;
+  if (!had_load_tile<kHad64TileBytes>(p.tile + (size_t)blockIdx.y * 343 * kFB, had32_dyn, &bar,
+                                      p.error, kMbarSpinLimit))
+    return;
+  const int chunk = blockIdx.x;
+  const int single = chunk - p.pairs.chunks, sparse = single - p.singles.chunks;
+  if (single < 0) had64_windows<2>(p, p.pairs, chunk, win, mem, had32_dyn);
+  else if (sparse < 0) had64_windows<1>(p, p.singles, single, win, mem, had32_dyn);
+  else had64_sparse(p, sparse, (const double2*)had32_dyn);
 }
 
 __global__ void __launch_bounds__(kHad32Threads, 1) hadamard_fp32_kernel(Had32Params p) {
@@ -1947,6 +2040,91 @@ __global__ void __launch_bounds__(kHadPairThreads, 1) hadamard_fp32_pair_kernel(
                         (float)(sums[(2 * c + 1) * 32] + ((double)hi_of(A[c]) + (double)lo_of(B[c]))));
     }
     __syncwarp();
+  }
+}
+
+// Sparse groups as in the FP64 form, two CTAs per SM; each 32 entries' FP32 sums
+// are added in FP64.
+constexpr int kHadSparseThreads = 256;
+constexpr int kHadSparseWarps = kHadSparseThreads / 32;
+
+struct HadSparse32Params {
+  int nn;
+  HadSparse sparse;
+  const float2* tile;
+  const float2* spec;
+  float2* effv;
+  int* error;
+  long long wait_limit;
+};
+
+__global__ void __launch_bounds__(kHadSparseThreads, 2)
+hadamard_fp32_sparse_kernel(HadSparse32Params p) {
+  extern __shared__ __align__(128) unsigned char had32_dyn[];
+  __shared__ __align__(8) unsigned long long bar;
+  const unsigned long long* tsm = (const unsigned long long*)had32_dyn;
+  const HadSparse& q = p.sparse;
+  const int f = threadIdx.x & 31, slot = threadIdx.x >> 5, chunk = blockIdx.x;
+  const size_t fbase = (size_t)blockIdx.y * p.nn;
+  if (!had_load_tile<kHad32TileBytes>(p.tile + (size_t)blockIdx.y * 343 * kFB, had32_dyn, &bar,
+                                      p.error, p.wait_limit))
+    return;
+  const unsigned long long* spec = (const unsigned long long*)p.spec + fbase * kFB + f;
+  const int g1 = min(q.n, (chunk + 1) * q.per_block);
+  for (int g = chunk * q.per_block + slot; g < g1; g += kHadSparseWarps) {
+    const int end = q.ptr[g + 1];
+    double ar[8], ai[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) ar[c] = ai[c] = 0.0;
+    for (int e0 = q.ptr[g]; e0 < end; e0 += 32) {
+      const int n = min(32, end - e0);
+      const int2 mine = f < n ? q.ent[e0 + f] : make_int2(0, 0);
+      unsigned long long A[8], B[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) A[c] = B[c] = 0ull;
+      constexpr int U = 4;
+      unsigned long long nxt[U];
+      auto fetch = [&](int i) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int node = __shfl_sync(0xffffffffu, mine.x, i + u);
+          nxt[u] = i + u < n ? spec[(size_t)node * kFB] : 0ull;
+        }
+      };
+      fetch(0);
+      for (int i = 0; i < n; i += U) {
+        unsigned long long sr[U], si[U];
+        const unsigned long long* t[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          sr[u] = pack2(lo_of(nxt[u]), lo_of(nxt[u]));
+          si[u] = pack2(hi_of(nxt[u]), hi_of(nxt[u]));
+          const int k = __shfl_sync(0xffffffffu, mine.y, i + u);
+          t[u] = tsm + (i + u < n ? k : had_member_offset(7)) * kFB + f;
+        }
+        if (i + U < n) fetch(i + U);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const unsigned long long w = t[u][-had_member_offset(c) * kFB];
+            asm("fma.rn.f32x2 %0, %2, %3, %0;\n"
+                "fma.rn.f32x2 %1, %2, %4, %1;\n"
+                : "+l"(A[c]), "+l"(B[c])
+                : "l"(w), "l"(sr[u]), "l"(si[u]));
+          }
+      }
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        ar[c] += (double)lo_of(A[c]) - (double)hi_of(B[c]);
+        ai[c] += (double)hi_of(A[c]) + (double)lo_of(B[c]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int m = q.members[(size_t)g * 8 + c];
+      if (m >= 0) p.effv[(fbase + m) * kFB + f] = make_float2((float)ar[c], (float)ai[c]);
+    }
   }
 }
 

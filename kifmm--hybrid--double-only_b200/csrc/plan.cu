@@ -118,7 +118,6 @@ struct kfmm_plan {
   // collects [0] over the kfmm_evaluate_async calls since the last wait
   int* d_error = nullptr;
   long long wait_limit = kMbarSpinLimit;  // tries of the V-list tile-copy wait
-  int single_per_block = 0, single_split = 1;  // Hadamard launch shapes (set_had_blocks)
   int p2p_grid = 0;            // resident P2P blocks on the device
   bool nf_minb5 = false;       // mixed near field with 5 resident blocks per SM
   kfmm_tuning tune{};          // launch choices asked for at creation (0 = automatic)
@@ -127,13 +126,8 @@ struct kfmm_plan {
   int *fft_nodes = nullptr, *ifft_nodes = nullptr;
   int n_fft = 0, n_ifft = 0;
   int n_groups = 0;
-  // x-neighbour pairs of sibling groups and the groups left single
-  unsigned long long* pair_rows = nullptr;  // per pair window: rows holding an entry
-  unsigned long long* single_rows = nullptr;
-  int *pair_win = nullptr, *pair_members = nullptr, *single_win = nullptr,
-      *single_members = nullptr;
-  int n_pairs = 0, n_singles = 0;
-  int pair_per_block = 0, pair_split = 1;
+  HadSet pairs, singles;  // x-neighbour pairs of sibling groups, the groups left single
+  HadSparse sparse;       // the groups taken entry by entry
   // tensor-core Hadamard (mixed form) on the complete levels it takes: levels,
   // box -> node maps and the MMAs' B operands; the spectra, the error flag and
   // the unit counter are filled in at launch
@@ -212,12 +206,14 @@ kfmm_status upload(kfmm_plan* p, T** ptr, const std::vector<T>& h) {
   } while (0)
 
 // Large tiles (160 x 64, kGemmRows x kGemmBN) when they give every SM its two
-// blocks; else small tiles, with the fewest column groups per CTA (the most
+// blocks and at least half of their rows are used (operators of at most 80 rows, NP
+// 3 and 4, take small tiles always: products of 4M points on the ellipsoid surface
+// 0.525 -> 0.510 ms); else small tiles, with the fewest column groups per CTA (the most
 // shares of K, up to the tuning's splitk_max) that leave at most two CTAs per SM.
 void choose_tiles(const kfmm_plan* p, GemmBatch& g) {
   const int want = 2 * p->num_sms;
   g.wn = 0;
-  if (g.chunks * ((g.ncol + kGemmBN - 1) / kGemmBN) >= want) return;
+  if (g.M > kGemmRows / 2 && g.chunks * ((g.ncol + kGemmBN - 1) / kGemmBN) >= want) return;
   const int mt = (g.M + kSmallRows - 1) / kSmallRows;
   auto ctas = [&](int wn) { return mt * ((g.ncol + kSmallCols * wn - 1) / (kSmallCols * wn)); };
   g.wn = 1;
@@ -231,7 +227,8 @@ void count_launches(kfmm_plan* p) {
   p->stats.tensor_levels = p->n_tc_levels;
   p->stats.host_pairs = p->host_pairs;
   p->stats.launches = (p->n_s2m > 0) + (int)p->up_gemms.size() + (p->n_fft > 0) +
-                      (p->n_pairs > 0) + (p->n_singles > 0) +
+                      (p->prec == KFMM_MIXED ? (p->pairs.nwin > 0) + (p->singles.nwin > 0) + (p->sparse.n > 0)
+                                             : (p->n_groups > 0)) +
                       (p->n_tc_levels > 0) + (p->n_ifft > 0) + (p->n_s2l > 0) +
                       (int)p->down_gemms.size() + (p->n_nf > 0);
 }
@@ -447,7 +444,8 @@ void add_part(std::vector<P2PJob>& jobs, const P2PJob& all, int from, int to) {
 void split_even(std::vector<P2PJob>& jobs, const P2PJob& all, int count, int rows) {
   const int full = (count + 31) / 32, parts = (full + rows - 1) / rows;
   for (int c = 0; c < parts; ++c)
-    add_part(jobs, all, 32 * (full * c / parts), std::min(count, 32 * (full * (c + 1) / parts)));
+    add_part(jobs, all, 32 * (int)((long long)full * c / parts),
+             std::min(count, 32 * (int)((long long)full * (c + 1) / parts)));
 }
 
 // One warp per job: parts of 32 * rows targets (rows: 0 for the automatic choice,
@@ -521,36 +519,50 @@ kfmm_status build_nf_jobs(kfmm_plan* p) {
 
 // Hadamard launch shapes: one CTA per SM over (chunks x frequency blocks).  A
 // chunk holds k windows per warp (every warp the same count, so none idles at
-// the end of its CTA); k minimises the span ceil(CTAs / SMs) x (k + tile), tile
-// standing for a CTA's translation-tile load (FP32 0.1, FP64 0.2 windows), unless
-// the tuning fixes k.  The FP64 kernel may also give a window to 2, 4 or 8 warps,
-// one window per team: k = 1 / split.
+// the end of its CTA), or one window per team of `split` warps (k = 1 / split); the
+// choice minimises the span ceil(CTAs / SMs) x (k + tile), tile standing for a
+// CTA's translation-tile load (FP32 0.1, FP64 0.2 windows).  The tuning may fix k
+// (mixed form) where windows are not shared: sharing changes a sum's order.
 void set_had_blocks(kfmm_plan* p) {
   const int nfb = p->Fpad / kFB;
   const bool mixed = p->prec == KFMM_MIXED;
-  auto shape = [&](int items, int warps, int* per, int* split) {
-    *split = 1;
-    if (p->tune.had_windows > 0 && mixed) {
-      *per = warps * std::min(p->tune.had_windows, 8);
-      return;
-    }
-    *per = warps;
+  auto span = [&](int chunks, int resident, double k) {
+    return std::ceil((double)chunks * nfb / (resident * p->num_sms)) * (k + (mixed ? 0.1 : 0.2));
+  };
+  for (HadSet* q : {&p->pairs, &p->singles}) {
+    const int warps = !mixed ? kHad64Warps : q == &p->pairs ? kHadPairWarps : kHad32Warps;
     double best = 1e300;
-    auto consider = [&](int windows, int s, double k) {
-      const long long ctas = (long long)((items + windows - 1) / windows) * nfb;
-      const double span = std::ceil((double)ctas / p->num_sms) * (k + (mixed ? 0.1 : 0.2));
-      if (span < best) {
-        best = span;
-        *per = windows;
-        *split = s;
+    auto consider = [&](int windows, int split, double k) {
+      const int chunks = (q->nwin + windows - 1) / windows;
+      const double t = span(chunks, 1, k);
+      if (t < best) {
+        best = t;
+        q->win_per_block = windows;
+        q->split = split;
+        q->chunks = chunks;
       }
     };
+    if (mixed && p->tune.had_windows > 0) {
+      consider(warps * std::min(p->tune.had_windows, 8), 1, 1.0);
+      continue;
+    }
     for (int k = 1; k <= 8; ++k) consider(warps * k, 1, k);
-    if (!mixed)
-      for (int s = 2; s <= warps; s *= 2) consider(warps / s, s, 1.0 / s);
-  };
-  shape(p->n_singles, mixed ? kHad32Warps : kHad64Warps, &p->single_per_block, &p->single_split);
-  shape(p->n_pairs, mixed ? kHadPairWarps : kHad64Warps, &p->pair_per_block, &p->pair_split);
+    for (int split = 2; split <= warps && !mixed; ++split)
+      if (warps % split == 0) consider(warps / split, split, 1.0 / split);
+  }
+  // sparse groups: a group takes about a third of a dense window's time
+  HadSparse& q = p->sparse;
+  const int warps = mixed ? kHadSparseWarps : kHad64Warps;
+  double best = 1e300;
+  for (int k = 1; k <= 16; ++k) {
+    const int chunks = (q.n + warps * k - 1) / (warps * k);
+    const double t = span(chunks, mixed ? 2 : 1, k / 3.0);
+    if (t < best) {
+      best = t;
+      q.per_block = warps * k;
+      q.chunks = chunks;
+    }
+  }
 }
 
 kfmm_status check_tuning(const kfmm_tuning* t) {
@@ -1022,6 +1034,37 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
       std::vector<char> used(p->n_groups, 0);
       for (int g = 0; g < p->n_groups; ++g) used[g] = tc_level[d->depth[gparent[g]] + 1];
       std::vector<int> pwin, pmem, swin, smem;
+      // Present entries of a group's window but for the eight boxes of the group
+      // itself, which are adjacent to every member, and the rows that hold any.
+      auto count = [&](int g, unsigned long long& rows) {
+        int n = 0;
+        for (int q = 0; q < 216; ++q) {
+          const int x = q % 6, y = q / 6 % 6, z = q / 36;
+          const bool own = (x == 2 || x == 3) && (y == 2 || y == 3) && (z == 2 || z == 3);
+          if (win[(size_t)g * 216 + q] < 0 || own) continue;
+          ++n;
+          rows |= 1ull << (y + 6 * z);
+        }
+        return n;
+      };
+      std::vector<int> sp_ptr(1, 0), sp_mem;
+      std::vector<int2> sp_ent;
+      auto add_sparse = [&](int g) {
+        for (int q = 0; q < 216; ++q) {
+          const int x = q % 6, y = q / 6 % 6, z = q / 36;
+          const bool own = (x == 2 || x == 3) && (y == 2 || y == 3) && (z == 2 || z == 3);
+          if (win[(size_t)g * 216 + q] < 0 || own) continue;
+          sp_ent.push_back(make_int2(win[(size_t)g * 216 + q], (x + 1) + 7 * (y + 1) + 49 * (z + 1)));
+        }
+        sp_ptr.push_back((int)sp_ent.size());
+        sp_mem.insert(sp_mem.end(), &mem[(size_t)g * 8], &mem[(size_t)g * 8] + 8);
+      };
+      // Entry by entry where a visited row holds fewer than 6 of a pair's 12 entries
+      // (both groups'), or fewer than 5 of a single group's 6.  Hadamard with limits
+      // none / (6, 4) / (8, 5): 4M points on the ellipsoid surface, NP 4, mixed 0.57 /
+      // 0.52 / 0.53 ms, plain 0.90 / 0.74 ms; 20,011 points on the ellipse, NP 3, mixed
+      // 65 / 30 / 21 us; 4M uniform, mixed 1.48 / 1.48 / 1.51 ms.
+      constexpr int kSparsePair = 6, kSparseSingle = 5;
       for (int g = 0; g < p->n_groups; ++g) {
         if (used[g]) continue;
         const int pn = gparent[g];
@@ -1032,6 +1075,20 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
           if (it != level.end() && !used[it->second]) partner = it->second;
         }
         used[g] = 1;
+        unsigned long long rows = 0ull;
+        const int entries = count(g, rows);
+        if (partner >= 0) {
+          const int both = entries + count(partner, rows);
+          if (both < kSparsePair * __builtin_popcountll(rows)) {
+            add_sparse(g);
+            add_sparse(partner);
+            used[partner] = 1;
+            continue;
+          }
+        } else if (entries < kSparseSingle * __builtin_popcountll(rows)) {
+          add_sparse(g);
+          continue;
+        }
         if (partner < 0) {
           swin.insert(swin.end(), &win[(size_t)g * 216], &win[(size_t)g * 216] + 216);
           smem.insert(smem.end(), &mem[(size_t)g * 8], &mem[(size_t)g * 8] + 8);
@@ -1053,26 +1110,45 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
         pmem.insert(pmem.end(), &mem[(size_t)g * 8], &mem[(size_t)g * 8] + 8);
         pmem.insert(pmem.end(), &mem[(size_t)partner * 8], &mem[(size_t)partner * 8] + 8);
       }
-      p->n_pairs = (int)pmem.size() / 16;
-      p->n_singles = (int)smem.size() / 8;
-      KF_TRY(upload(p, &p->pair_win, pwin));
+      p->pairs.nwin = (int)pmem.size() / 16;
+      p->singles.nwin = (int)smem.size() / 8;
+      int *pw = nullptr, *pm = nullptr, *sw = nullptr, *sm = nullptr;
+      unsigned long long *pr = nullptr, *sr = nullptr;
+      KF_TRY(upload(p, &pw, pwin));
       {
         std::vector<unsigned long long> prow(pmem.size() / 16, 0ull);
         for (size_t g = 0; g < prow.size(); ++g)
           for (int r = 0; r < 36; ++r)
             for (int x = 0; x < 8; ++x)
               if (pwin[g * 288 + r * 8 + x] >= 0) prow[g] |= 1ull << r;
-        KF_TRY(upload(p, &p->pair_rows, prow));
+        KF_TRY(upload(p, &pr, prow));
         std::vector<unsigned long long> srow(smem.size() / 8, 0ull);
         for (size_t g = 0; g < srow.size(); ++g)
           for (int r = 0; r < 36; ++r)
             for (int x = 0; x < 6; ++x)
               if (swin[g * 216 + r * 6 + x] >= 0) srow[g] |= 1ull << r;
-        KF_TRY(upload(p, &p->single_rows, srow));
+        KF_TRY(upload(p, &sr, srow));
       }
-      KF_TRY(upload(p, &p->pair_members, pmem));
-      KF_TRY(upload(p, &p->single_win, swin));
-      KF_TRY(upload(p, &p->single_members, smem));
+      KF_TRY(upload(p, &pm, pmem));
+      KF_TRY(upload(p, &sw, swin));
+      KF_TRY(upload(p, &sm, smem));
+      p->sparse.n = (int)sp_mem.size() / 8;
+      if (p->sparse.n) {
+        int *sp = nullptr, *spm = nullptr;
+        int2* se = nullptr;
+        KF_TRY(upload(p, &sp, sp_ptr));
+        KF_TRY(upload(p, &se, sp_ent));
+        KF_TRY(upload(p, &spm, sp_mem));
+        p->sparse.ptr = sp;
+        p->sparse.ent = se;
+        p->sparse.members = spm;
+      }
+      p->pairs.win = pw;
+      p->pairs.members = pm;
+      p->pairs.rows = pr;
+      p->singles.win = sw;
+      p->singles.members = sm;
+      p->singles.rows = sr;
     }
     p->stats.spectra_bytes = 16.0 * F * ((double)fn.size() + (double)ifn.size());
   }
@@ -1243,13 +1319,13 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
                                (int)kTcSmemBytes));
   KF_CUDA(cudaFuncSetAttribute(hadamard_fp32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kHad32TileBytes));
-  KF_CUDA(cudaFuncSetAttribute(hadamard_fp64_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)kHad64TileBytes));
-  KF_CUDA(cudaFuncSetAttribute(hadamard_fp64_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)kHad64TileBytes));
+  KF_CUDA(cudaFuncSetAttribute(hadamard_fp32_sparse_kernel,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHad32TileBytes));
   KF_CUDA(cudaFuncSetAttribute(hadamard_fp32_pair_kernel,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kHadPairSmemBytes));
+  KF_CUDA(cudaFuncSetAttribute(hadamard_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kHad64TileBytes));
   set_had_blocks(p);
 
   KF_TRY(dalloc(p, &p->job_counter, 3));
@@ -1550,23 +1626,30 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
   mark(p, 3, S(stream));
   if (p->n_groups) {
     if (mixed) {
-      if (p->n_pairs) {
-        const int ppb = p->pair_per_block;
-        HadPairParams h{p->nn, p->n_pairs, ppb, p->pair_win, p->pair_members, p->pair_rows,
+      const int nfb = p->Fpad / kFB;
+      if (p->pairs.nwin) {
+        const HadSet& q = p->pairs;
+        HadPairParams h{p->nn, q.nwin, q.win_per_block, q.win, q.members, q.rows,
                         (const float2*)p->d_trans, (const float2*)p->spec, (float2*)p->effv,
                         p->d_error, p->wait_limit};
-        dim3 grid((p->n_pairs + ppb - 1) / ppb, p->Fpad / kFB);
-        hadamard_fp32_pair_kernel<<<grid, kHadPairThreads, kHadPairSmemBytes, S(stream)>>>(h);
+        hadamard_fp32_pair_kernel<<<dim3(q.chunks, nfb), kHadPairThreads, kHadPairSmemBytes,
+                                    S(stream)>>>(h);
         KF_CHECK_LAUNCH("hadamard_fp32_pair_kernel");
       }
-      if (p->n_singles) {
-        const int gpb = p->single_per_block;
-        Had32Params h{p->nn, p->n_singles, gpb, p->single_win, p->single_members, p->single_rows,
+      if (p->singles.nwin) {
+        const HadSet& q = p->singles;
+        Had32Params h{p->nn, q.nwin, q.win_per_block, q.win, q.members, q.rows,
                       (const float2*)p->d_trans, (const float2*)p->spec, (float2*)p->effv,
                       p->d_error, p->wait_limit};
-        dim3 grid((p->n_singles + gpb - 1) / gpb, p->Fpad / kFB);
-        hadamard_fp32_kernel<<<grid, kHad32Threads, kHad32TileBytes, S(stream)>>>(h);
+        hadamard_fp32_kernel<<<dim3(q.chunks, nfb), kHad32Threads, kHad32TileBytes, S(stream)>>>(h);
         KF_CHECK_LAUNCH("hadamard_fp32_kernel");
+      }
+      if (p->sparse.n) {
+        HadSparse32Params h{p->nn, p->sparse, (const float2*)p->d_trans, (const float2*)p->spec,
+                            (float2*)p->effv, p->d_error, p->wait_limit};
+        hadamard_fp32_sparse_kernel<<<dim3(p->sparse.chunks, nfb), kHadSparseThreads,
+                                      kHad32TileBytes, S(stream)>>>(h);
+        KF_CHECK_LAUNCH("hadamard_fp32_sparse_kernel");
       }
       if (p->n_tc_levels) {
         KF_CUDA(cudaMemsetAsync(p->tc_counter, 0, sizeof(int), S(stream)));
@@ -1580,18 +1663,10 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
         KF_CHECK_LAUNCH("hadamard_tc_kernel");
       }
     } else {
-      auto launch = [&](auto kern, int nwin, int per, int split, const int* win, const int* members,
-                        const unsigned long long* rows) {
-        if (nwin == 0) return;
-        Had64Params h{p->nn, nwin, per, split, win, members, rows, (const double2*)p->d_trans,
-                      (const double2*)p->spec, (double2*)p->effv, p->d_error};
-        dim3 grid((nwin + per - 1) / per, p->Fpad / kFB);
-        kern<<<grid, kHad64Threads, kHad64TileBytes, S(stream)>>>(h);
-      };
-      launch(hadamard_fp64_kernel<2>, p->n_pairs, p->pair_per_block, p->pair_split, p->pair_win,
-             p->pair_members, p->pair_rows);
-      launch(hadamard_fp64_kernel<1>, p->n_singles, p->single_per_block, p->single_split,
-             p->single_win, p->single_members, p->single_rows);
+      Had64Params h{p->nn, p->pairs, p->singles, p->sparse, (const double2*)p->d_trans,
+                    (const double2*)p->spec, (double2*)p->effv, p->d_error};
+      const dim3 grid(p->pairs.chunks + p->singles.chunks + p->sparse.chunks, p->Fpad / kFB);
+      hadamard_fp64_kernel<<<grid, kHad64Threads, kHad64TileBytes, S(stream)>>>(h);
       KF_CHECK_LAUNCH("hadamard_fp64_kernel");
     }
   }
