@@ -2169,6 +2169,12 @@ __global__ void error_fold_kernel(int* error) {
   if (error[0]) error[1] = 1;
 }
 
+// The error flags of a batch's plans, side by side.
+__global__ void gather_flags_kernel(int n, const int* const* flags, int* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = *flags[i];
+}
+
 // Direct sum (ulist__direct_evaluation) over SoA device arrays, any coordinates.
 // Bound by the FP64 pipe (12 operations a pair, pair_rsqrt).  A warp takes 32
 // targets, one per lane, and every (kSplit x cluster size)-th chunk of 32 sources,

@@ -19,6 +19,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <unordered_map>
@@ -64,6 +65,50 @@ struct GemmBatch {
   int ncol;
   int accumulate;
 };
+
+// Pinned slots of two ints in which the plans' error flags land on the host.  A
+// copy to pageable memory costs a staging pass and a wait of its own (about 8 us of
+// every solve handed back), and a pinned allocation per plan costs more than
+// creating a small plan (4,096 points: 3 -> 13 ms), so plans share one page of
+// slots, allocated with the first plan and kept; a plan that finds none free reads
+// its flags through pageable memory.  A page lost to a device reset is replaced.
+class FlagSlots {
+ public:
+  int* take() {
+    std::lock_guard<std::mutex> lock(mu_);
+    cudaPointerAttributes at{};
+    if (base_ &&
+        (cudaPointerGetAttributes(&at, base_) != cudaSuccess || at.type != cudaMemoryTypeHost)) {
+      cudaGetLastError();
+      base_ = nullptr;
+    }
+    if (!base_) {
+      void* v = nullptr;
+      if (cudaHostAlloc(&v, sizeof(int) * 2 * kSlots, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+      }
+      base_ = (int*)v;
+      free_.clear();
+      for (int i = kSlots - 1; i >= 0; --i) free_.push_back(base_ + 2 * i);
+    }
+    if (free_.empty()) return nullptr;
+    int* s = free_.back();
+    free_.pop_back();
+    return s;
+  }
+  void give(int* s) {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (s && base_ && s >= base_ && s < base_ + 2 * kSlots) free_.push_back(s);
+  }
+
+ private:
+  static constexpr int kSlots = 512;  // 4 KiB
+  std::mutex mu_;
+  int* base_ = nullptr;
+  std::vector<int*> free_;
+};
+static FlagSlots g_flag_slots;
 
 }  // namespace kfmm
 
@@ -117,6 +162,7 @@ struct kfmm_plan {
   // [0] set by kernels whose bounded waits ran out, zeroed per solve; [1]
   // collects [0] over the kfmm_evaluate_async calls since the last wait
   int* d_error = nullptr;
+  int* h_error = nullptr;  // where the host reads the two (a slot of g_flag_slots)
   long long wait_limit = kMbarSpinLimit;  // tries of the V-list tile-copy wait
   int p2p_grid = 0;            // resident P2P blocks on the device
   bool nf_minb5 = false;       // mixed near field with 5 resident blocks per SM
@@ -1331,6 +1377,7 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
   KF_TRY(dalloc(p, &p->job_counter, 3));
   KF_TRY(dalloc(p, &p->d_error, 2));
   KF_CUDA(cudaMemset(p->d_error, 0, 2 * sizeof(int)));
+  p->h_error = g_flag_slots.take();
   p->stats.num_nodes = nn;
   p->stats.P = P;
   p->stats.Q = Q;
@@ -1442,10 +1489,11 @@ void mark(kfmm_plan* p, int i, cudaStream_t st) {
 // Waits for `stream` and reports whether a kernel of the plan's last solve
 // gave up a bounded wait (the flag is zeroed at the start of every V list).
 kfmm_status sync_and_check(kfmm_plan* p, cudaStream_t st) {
-  int err = 0;
-  KF_CUDA(cudaMemcpyAsync(&err, p->d_error, sizeof(int), cudaMemcpyDeviceToHost, st));
+  int pageable[2] = {0, 0};
+  int* err = p->h_error ? p->h_error : pageable;
+  KF_CUDA(cudaMemcpyAsync(err, p->d_error, sizeof(int), cudaMemcpyDeviceToHost, st));
   KF_CUDA(cudaStreamSynchronize(st));
-  if (err) {
+  if (err[0]) {
     set_error("a kernel's bounded wait ran out (V-list translation tile copy)");
     return KFMM_ERR_CUDA;
   }
@@ -1506,6 +1554,7 @@ kfmm_status kfmm_plan_create_tuned(const kfmm_tree_desc* tree, int np, kfmm_prec
 kfmm_status kfmm_plan_destroy(kfmm_plan* p) {
   if (!p) return KFMM_OK;
   for (void* v : p->allocs) cudaFree(v);
+  g_flag_slots.give(p->h_error);
   for (int i = 0; i < kfmm_plan::kMarks; ++i)
     if (p->ev[i]) cudaEventDestroy(p->ev[i]);
   for (cudaEvent_t e : {p->ev_h2d_src, p->ev_gsrc, p->ev_gtrg, p->ev_nf, p->ev_d2h})
@@ -1884,7 +1933,8 @@ kfmm_status kfmm_evaluate_join(kfmm_plan* p, void* stream) {
 
 kfmm_status kfmm_evaluate_wait(kfmm_plan* p, void* stream) {
   KF_TRY(kfmm_evaluate_join(p, stream));
-  int err[2] = {0, 0};
+  int pageable[2] = {0, 0};
+  int* err = p->h_error ? p->h_error : pageable;
   KF_CUDA(cudaMemcpyAsync(err, p->d_error, 2 * sizeof(int), cudaMemcpyDeviceToHost, S(stream)));
   KF_CUDA(cudaStreamSynchronize(S(stream)));
   if (err[1]) {
@@ -2012,7 +2062,10 @@ struct kfmm_batch {
   void* d_params = nullptr;  // P2PMixedParams (mixed plans) or P2PParams
   P2PJob* d_jobs = nullptr;  // team jobs, then one-warp jobs
   int* d_counter = nullptr;
-  std::vector<kfmm_plan*> plans;  // for the error flags kfmm_batch_wait reads
+  // the plans' error flags, gathered by the graph's last node for kfmm_batch_wait
+  const int** d_flags = nullptr;
+  int* d_gathered = nullptr;
+  int nplans = 0;
 };
 
 static void batch_release(kfmm_batch* b) {
@@ -2022,6 +2075,8 @@ static void batch_release(kfmm_batch* b) {
   if (b->d_params) cudaFree(b->d_params);
   if (b->d_jobs) cudaFree(b->d_jobs);
   if (b->d_counter) cudaFree(b->d_counter);
+  if (b->d_flags) cudaFree(b->d_flags);
+  if (b->d_gathered) cudaFree(b->d_gathered);
   for (cudaEvent_t e : b->events) cudaEventDestroy(e);
   for (cudaStream_t s : b->streams) cudaStreamDestroy(s);
   delete b;
@@ -2043,7 +2098,7 @@ kfmm_status kfmm_batch_create(kfmm_plan* const* plans, int nplans, int nstreams,
   }
   nstreams = std::min(nstreams, nplans);
   kfmm_batch* b = new kfmm_batch();
-  b->plans.assign(plans, plans + nplans);
+  b->nplans = nplans;
   auto fail = [&](cudaError_t e, const char* what) {
     set_error(std::string("kfmm_batch_create: ") + what + ": " + cudaGetErrorString(e));
     batch_release(b);
@@ -2111,6 +2166,15 @@ kfmm_status kfmm_batch_create(kfmm_plan* const* plans, int nplans, int nstreams,
         (e = cudaMemcpy(b->d_jobs, jobs.data(), jbytes, cudaMemcpyHostToDevice)) != cudaSuccess)
       return fail(e, "cudaMemcpy");
   }
+  {
+    std::vector<const int*> flags(nplans);
+    for (int i = 0; i < nplans; ++i) flags[i] = plans[i]->d_error;
+    const size_t fbytes = sizeof(int*) * nplans;
+    if ((e = cudaMalloc((void**)&b->d_flags, fbytes)) != cudaSuccess ||
+        (e = cudaMalloc((void**)&b->d_gathered, sizeof(int) * nplans)) != cudaSuccess ||
+        (e = cudaMemcpy(b->d_flags, flags.data(), fbytes, cudaMemcpyHostToDevice)) != cudaSuccess)
+      return fail(e, "error flags");
+  }
   cudaStream_t origin = b->streams[nstreams];
   if ((e = cudaStreamBeginCapture(origin, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
     return fail(e, "cudaStreamBeginCapture");
@@ -2154,6 +2218,13 @@ kfmm_status kfmm_batch_create(kfmm_plan* const* plans, int nplans, int nstreams,
       st = KFMM_ERR_CUDA;
     }
   }
+  if (st == KFMM_OK) {
+    gather_flags_kernel<<<(nplans + 127) / 128, 128, 0, origin>>>(nplans, b->d_flags, b->d_gathered);
+    if (cudaGetLastError() != cudaSuccess) {
+      set_error("kfmm_batch_create: error-flag launch failed");
+      st = KFMM_ERR_CUDA;
+    }
+  }
   e = cudaStreamEndCapture(origin, &b->graph);
   if (st != KFMM_OK) {
     batch_release(b);
@@ -2180,10 +2251,9 @@ kfmm_status kfmm_batch_wait(kfmm_batch* b, void* stream) {
     set_error("kfmm_batch_wait: null batch");
     return KFMM_ERR_INVALID;
   }
-  std::vector<int> err(b->plans.size(), 0);
-  for (size_t i = 0; i < b->plans.size(); ++i)
-    KF_CUDA(cudaMemcpyAsync(&err[i], b->plans[i]->d_error, sizeof(int), cudaMemcpyDeviceToHost,
-                            S(stream)));
+  std::vector<int> err(b->nplans, 0);
+  KF_CUDA(cudaMemcpyAsync(err.data(), b->d_gathered, sizeof(int) * err.size(),
+                          cudaMemcpyDeviceToHost, S(stream)));
   KF_CUDA(cudaStreamSynchronize(S(stream)));
   for (size_t i = 0; i < err.size(); ++i)
     if (err[i]) {
