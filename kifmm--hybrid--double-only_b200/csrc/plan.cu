@@ -195,6 +195,7 @@ struct kfmm_plan {
   kfmm_stats stats{};
   int num_sms = 148;
   bool timing = false;
+  bool chained = true;  // far-field launches as programmatic dependents; not in batches
   // timing marks (kfmm_enable_timing): 0 start, 1 S2M pairs done, 2 up done,
   // 3 forward FFT, 4 Hadamard, 5 inverse FFT (V done), 6 S2L (X done),
   // 7 down done, 8 near field done, 9 copy done
@@ -268,6 +269,24 @@ void choose_tiles(const kfmm_plan* p, GemmBatch& g) {
   while (g.wn < kSmallWarps && ctas(g.wn) > want) g.wn *= 2;
 }
 
+// Launches a kernel of the far field: with `chained`, its blocks may start before
+// the kernel before it on the stream is done (they wait in chain_wait).
+template <class... P, class... A>
+cudaError_t launch_chained(bool chained, void (*kern)(P...), dim3 grid, int threads, size_t smem,
+                           cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = chained ? 1 : 0;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 // Kernel launches of one kfmm_run (kfmm_plan_stats.launches).
 void count_launches(kfmm_plan* p) {
   p->stats.tensor_levels = p->n_tc_levels;
@@ -317,15 +336,15 @@ kfmm_status launch_gemms(const kfmm_plan* p, const std::vector<GemmBatch>& gs, c
     if (b.wn) {
       const int cols = kSmallCols * b.wn;
       dim3 grid((b.M + kSmallRows - 1) / kSmallRows, (b.ncol + cols - 1) / cols);
-      gemm_fp64_small_kernel<<<grid, 32 * kSmallWarps, 0, st>>>(a, b.wn);
+      launch_chained(p->chained, gemm_fp64_small_kernel, grid, 32 * kSmallWarps, 0, st, a, b.wn);
       KF_CHECK_LAUNCH("gemm_fp64_small_kernel");
       continue;
     }
     dim3 grid(b.chunks, (b.ncol + kGemmBN - 1) / kGemmBN);
     if (b.accumulate)
-      gemm_fp64_dmma_kernel<true><<<grid, kGemmThreads, kGemmSmemBytes, st>>>(a, b.mrows);
+      launch_chained(p->chained, gemm_fp64_dmma_kernel<true>, grid, kGemmThreads, kGemmSmemBytes, st, a, b.mrows);
     else
-      gemm_fp64_dmma_kernel<false><<<grid, kGemmThreads, kGemmSmemBytes, st>>>(a, b.mrows);
+      launch_chained(p->chained, gemm_fp64_dmma_kernel<false>, grid, kGemmThreads, kGemmSmemBytes, st, a, b.mrows);
     KF_CHECK_LAUNCH("gemm_fp64_dmma_kernel");
   }
   return KFMM_OK;
@@ -1424,7 +1443,7 @@ int fft_src_resident(int np, bool mixed) {
 }
 
 template <int NP>
-void fft_launch_np(bool mixed, bool forward, int nboxes, int num_sms, FFTParams f,
+void fft_launch_np(bool chained, bool mixed, bool forward, int nboxes, int num_sms, FFTParams f,
                    cudaStream_t st) {
   constexpr int B = fft_boxes_per_block<NP>();
   const int nblocks = (nboxes + B - 1) / B;
@@ -1432,23 +1451,25 @@ void fft_launch_np(bool mixed, bool forward, int nboxes, int num_sms, FFTParams 
   if (forward) {
     // persistent: one wave of blocks, each taking groups of boxes in turn
     const int grid = std::max(1, std::min(nblocks, num_sms * fft_src_resident<NP>(mixed)));
-    if (mixed) fft_src_np_kernel<NP, float2><<<grid, kFFTThreads, 0, st>>>(f);
-    else fft_src_np_kernel<NP, double2><<<grid, kFFTThreads, 0, st>>>(f);
+    if (mixed) launch_chained(chained, fft_src_np_kernel<NP, float2>, grid, kFFTThreads, 0, st, f);
+    else launch_chained(chained, fft_src_np_kernel<NP, double2>, grid, kFFTThreads, 0, st, f);
   } else {
-    if (mixed) ifft_trg_np_kernel<NP, float2><<<nblocks, kFFTThreads, 0, st>>>(f);
-    else ifft_trg_np_kernel<NP, double2><<<nblocks, kFFTThreads, 0, st>>>(f);
+    if (mixed) launch_chained(chained, ifft_trg_np_kernel<NP, float2>, nblocks, kFFTThreads, 0, st, f);
+    else launch_chained(chained, ifft_trg_np_kernel<NP, double2>, nblocks, kFFTThreads, 0, st, f);
   }
 }
 
-kfmm_status launch_fft(int np, bool mixed, bool forward, int nboxes, int num_sms,
-                       const FFTParams& f, void* stream) {
-  switch (np) {
-    case 3: fft_launch_np<3>(mixed, forward, nboxes, num_sms, f, S(stream)); break;
-    case 4: fft_launch_np<4>(mixed, forward, nboxes, num_sms, f, S(stream)); break;
-    case 5: fft_launch_np<5>(mixed, forward, nboxes, num_sms, f, S(stream)); break;
-    case 6: fft_launch_np<6>(mixed, forward, nboxes, num_sms, f, S(stream)); break;
-    case 7: fft_launch_np<7>(mixed, forward, nboxes, num_sms, f, S(stream)); break;
-    case 8: fft_launch_np<8>(mixed, forward, nboxes, num_sms, f, S(stream)); break;
+kfmm_status launch_fft(const kfmm_plan* p, bool forward, int nboxes, const FFTParams& f,
+                       void* stream) {
+  const bool mixed = p->prec == KFMM_MIXED;
+  const int num_sms = p->num_sms;
+  switch (p->np) {
+    case 3: fft_launch_np<3>(p->chained, mixed, forward, nboxes, num_sms, f, S(stream)); break;
+    case 4: fft_launch_np<4>(p->chained, mixed, forward, nboxes, num_sms, f, S(stream)); break;
+    case 5: fft_launch_np<5>(p->chained, mixed, forward, nboxes, num_sms, f, S(stream)); break;
+    case 6: fft_launch_np<6>(p->chained, mixed, forward, nboxes, num_sms, f, S(stream)); break;
+    case 7: fft_launch_np<7>(p->chained, mixed, forward, nboxes, num_sms, f, S(stream)); break;
+    case 8: fft_launch_np<8>(p->chained, mixed, forward, nboxes, num_sms, f, S(stream)); break;
     default: set_error("launch_fft: NP out of range"); return KFMM_ERR_UNSUPPORTED;
   }
   KF_CHECK_LAUNCH(forward ? "fft_src_np_kernel" : "ifft_trg_np_kernel");
@@ -1660,9 +1681,12 @@ kfmm_status kfmm_up_calc(kfmm_plan* p, void* stream) {
 
 kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
   if (!p) return KFMM_ERR_INVALID;
-  // the error flag reports this solve's waits only
-  KF_CUDA(cudaMemsetAsync(p->d_error, 0, sizeof(int), S(stream)));
-  KF_CUDA(cudaMemsetAsync(p->dchk, 0, sizeof(double) * (size_t)p->nn * p->P, S(stream)));
+  // the error flag reports this solve's waits only; with sources to transform the
+  // forward transform zeroes both
+  if (!p->n_fft) {
+    KF_CUDA(cudaMemsetAsync(p->d_error, 0, sizeof(int), S(stream)));
+    KF_CUDA(cudaMemsetAsync(p->dchk, 0, sizeof(double) * (size_t)p->nn * p->P, S(stream)));
+  }
   mark(p, 2, S(stream));
   FFTParams f = fft_params(p);
   const bool mixed = p->prec == KFMM_MIXED;
@@ -1670,7 +1694,9 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
     f.nodes = p->fft_nodes;
     f.pln = p->uden;
     f.specout = p->spec;
-    KF_TRY(launch_fft(p->np, mixed, true, p->n_fft, p->num_sms, f, stream));
+    f.zero = p->dchk;
+    f.error = p->d_error;
+    KF_TRY(launch_fft(p, true, p->n_fft, f, stream));
   }
   mark(p, 3, S(stream));
   if (p->n_groups) {
@@ -1681,8 +1707,7 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
         HadPairParams h{p->nn, q.nwin, q.win_per_block, q.win, q.members, q.rows,
                         (const float2*)p->d_trans, (const float2*)p->spec, (float2*)p->effv,
                         p->d_error, p->wait_limit};
-        hadamard_fp32_pair_kernel<<<dim3(q.chunks, nfb), kHadPairThreads, kHadPairSmemBytes,
-                                    S(stream)>>>(h);
+        launch_chained(p->chained, hadamard_fp32_pair_kernel, dim3(q.chunks, nfb), kHadPairThreads, kHadPairSmemBytes, S(stream), h);
         KF_CHECK_LAUNCH("hadamard_fp32_pair_kernel");
       }
       if (p->singles.nwin) {
@@ -1690,14 +1715,13 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
         Had32Params h{p->nn, q.nwin, q.win_per_block, q.win, q.members, q.rows,
                       (const float2*)p->d_trans, (const float2*)p->spec, (float2*)p->effv,
                       p->d_error, p->wait_limit};
-        hadamard_fp32_kernel<<<dim3(q.chunks, nfb), kHad32Threads, kHad32TileBytes, S(stream)>>>(h);
+        launch_chained(p->chained, hadamard_fp32_kernel, dim3(q.chunks, nfb), kHad32Threads, kHad32TileBytes, S(stream), h);
         KF_CHECK_LAUNCH("hadamard_fp32_kernel");
       }
       if (p->sparse.n) {
         HadSparse32Params h{p->nn, p->sparse, (const float2*)p->d_trans, (const float2*)p->spec,
                             (float2*)p->effv, p->d_error, p->wait_limit};
-        hadamard_fp32_sparse_kernel<<<dim3(p->sparse.chunks, nfb), kHadSparseThreads,
-                                      kHad32TileBytes, S(stream)>>>(h);
+        launch_chained(p->chained, hadamard_fp32_sparse_kernel, dim3(p->sparse.chunks, nfb), kHadSparseThreads, kHad32TileBytes, S(stream), h);
         KF_CHECK_LAUNCH("hadamard_fp32_sparse_kernel");
       }
       if (p->n_tc_levels) {
@@ -1715,7 +1739,7 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
       Had64Params h{p->nn, p->pairs, p->singles, p->sparse, (const double2*)p->d_trans,
                     (const double2*)p->spec, (double2*)p->effv, p->d_error};
       const dim3 grid(p->pairs.chunks + p->singles.chunks + p->sparse.chunks, p->Fpad / kFB);
-      hadamard_fp64_kernel<<<grid, kHad64Threads, kHad64TileBytes, S(stream)>>>(h);
+      launch_chained(p->chained, hadamard_fp64_kernel, grid, kHad64Threads, kHad64TileBytes, S(stream), h);
       KF_CHECK_LAUNCH("hadamard_fp64_kernel");
     }
   }
@@ -1724,7 +1748,7 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
     f.nodes = p->ifft_nodes;
     f.specin = p->effv;
     f.plnout = p->dchk;
-    KF_TRY(launch_fft(p->np, mixed, false, p->n_ifft, p->num_sms, f, stream));
+    KF_TRY(launch_fft(p, false, p->n_ifft, f, stream));
   }
   return KFMM_OK;
 }
@@ -2194,9 +2218,13 @@ kfmm_status kfmm_batch_create(kfmm_plan* const* plans, int nplans, int nstreams,
   for (int i = 0; i < nplans && st == KFMM_OK; ++i) {
     const bool timing = plans[i]->timing;
     plans[i]->timing = false;
+    // branches run side by side: waiting blocks of one would hold the others' slots
+    // (32 solves 2.22 -> 2.35 ms)
+    plans[i]->chained = false;
     cudaStream_t on = single ? origin : b->streams[i % nstreams];
     st = fused ? run_far_field(plans[i], on) : kfmm_run(plans[i], on);
     plans[i]->timing = timing;
+    plans[i]->chained = true;
   }
   if (!single) join();
   if (fused && st == KFMM_OK) {
