@@ -1011,88 +1011,84 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_fp64_dmma_kernel(GemmArg
 }
 
 // The same product in small tiles, operands straight from global memory (L2)
-// into the fragments: a CTA computes 40 rows x 16 wn columns, its 8 warps being wn
+// into the fragments: a CTA computes 32 rows x 16 wn columns, its 8 warps being wn
 // column groups times wk = 8 / wn shares of K, whose sums meet in shared memory.
 // No pipeline to fill, no split-K pass: what bounds a level product of a few
-// hundred columns is the latency of its start and of the passes after it.
-constexpr int kSmallRows = 40, kSmallCols = 16, kSmallWarps = 8;
-constexpr int kSmallOut = kSmallRows * kSmallCols;  // outputs of one warp tile
+// hundred columns is the latency of its start and of the passes after it; with
+// more columns it is the L1's rate, so the fragments are read 16 bytes a lane: a
+// load of A holds rows 2r and 2r + 1 of one k (rows of two m8 tiles), a load of B
+// holds k 2c and 2c + 1 of one column (two k steps, of the even and the odd k).
+constexpr int kSmallRows = 32, kSmallCols = 16, kSmallWarps = 8;
+constexpr int kSmallStride = kSmallRows + 2;
 
 __global__ void __launch_bounds__(32 * kSmallWarps, 2) gemm_fp64_small_kernel(GemmArgs g, int wn) {
-  __shared__ double red[kSmallWarps][kSmallOut];  // [warp][col][row]
+  __shared__ double red[kSmallWarps][kSmallCols * kSmallStride];  // [warp][col][row]
   chain_release();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wk = kSmallWarps / wn, cg = warp % wn, ks = warp / wn;
   const int m0 = blockIdx.x * kSmallRows, n0 = blockIdx.y * (kSmallCols * wn);
   const int r = lane >> 2, c = lane & 3;
-  // this warp's K range, a multiple of 4 but for the end
-  const int quads = (g.K + 3) / 4;
-  const int k0 = 4 * (quads * ks / wk), k1 = min(g.K, 4 * (quads * (ks + 1) / wk));
-  const double* ap[5];
+  // this warp's K range, a multiple of 8 but for the end
+  const int eights = (g.K + 7) / 8;
+  const int k0 = 8 * (eights * ks / wk), k1 = min(g.K, 8 * (eights * (ks + 1) / wk));
+  const double* ap[2];
 #pragma unroll
-  for (int i = 0; i < 5; ++i)  // rows beyond the matrix repeat its last (not stored)
-    ap[i] = g.A + (size_t)(k0 + c) * g.M + min(g.M - 1, m0 + 8 * i + r);
+  for (int i = 0; i < 2; ++i)  // rows beyond the matrix repeat its last two (not stored)
+    ap[i] = g.A + (size_t)(k0 + 2 * c) * g.M + min(g.M - 2, m0 + 16 * i + 2 * r);
   const double* bp[2];
 #pragma unroll
   for (int j = 0; j < 2; ++j)
-    bp[j] = g.B + g.boff[min(g.ncol - 1, n0 + cg * kSmallCols + 8 * j + r)] + k0 + c;
-  double acc[5][2][2];
+    bp[j] = g.B + g.boff[min(g.ncol - 1, n0 + cg * kSmallCols + 8 * j + r)] + k0 + 2 * c;
+  double acc[4][2][2];
 #pragma unroll
-  for (int i = 0; i < 5; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
   chain_wait();
-  int k = k0;
-  constexpr int U = 4;
-  for (; k + 4 * U <= k1; k += 4 * U) {
-    double af[U][5], bf[U][2];
+  constexpr int U = 2;  // eights of K in flight
+  for (int k = k0; k < k1; k += 8 * U) {
+    double2 af[U][2][2], bf[U][2];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
+      const bool in = k + 8 * u + 2 * c < k1;  // K is even
 #pragma unroll
-      for (int i = 0; i < 5; ++i) af[u][i] = __ldg(ap[i] + (size_t)(4 * u) * g.M);
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int j = 0; j < 2; ++j) bf[u][j] = bp[j][4 * u];
+        for (int i = 0; i < 2; ++i)
+          af[u][j][i] = in ? __ldg((const double2*)(ap[i] + (size_t)(8 * u + j) * g.M))
+                           : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        bf[u][j] = in ? *(const double2*)(bp[j] + 8 * u) : make_double2(0.0, 0.0);
     }
 #pragma unroll
-    for (int i = 0; i < 5; ++i) ap[i] += (size_t)(4 * U) * g.M;
+    for (int i = 0; i < 2; ++i) ap[i] += (size_t)(8 * U) * g.M;
 #pragma unroll
-    for (int j = 0; j < 2; ++j) bp[j] += 4 * U;
+    for (int j = 0; j < 2; ++j) bp[j] += 8 * U;
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int i = 0; i < 5; ++i)
+      for (int o = 0; o < 2; ++o)
 #pragma unroll
-        for (int j = 0; j < 2; ++j) dmma_884(acc[i][j][0], acc[i][j][1], af[u][i], bf[u][j]);
-  }
-  if (k < k1) {  // up to 15 more, zero beyond the range
-    double af[U][5], bf[U][2];
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const bool in = k + 4 * u + c < k1;
-#pragma unroll
-      for (int i = 0; i < 5; ++i) af[u][i] = in ? __ldg(ap[i] + (size_t)(4 * u) * g.M) : 0.0;
-#pragma unroll
-      for (int j = 0; j < 2; ++j) bf[u][j] = in ? bp[j][4 * u] : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int i = 0; i < 5; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) dmma_884(acc[i][j][0], acc[i][j][1], af[u][i], bf[u][j]);
+          for (int j = 0; j < 2; ++j)
+            dmma_884(acc[i][j][0], acc[i][j][1], i & 1 ? af[u][o][i >> 1].y : af[u][o][i >> 1].x,
+                     o ? bf[u][j].y : bf[u][j].x);
   }
 #pragma unroll
-  for (int i = 0; i < 5; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
       for (int h = 0; h < 2; ++h)
-        red[warp][(8 * j + 2 * c + h) * kSmallRows + 8 * i + r] = acc[i][j][h];
+        red[warp][(8 * j + 2 * c + h) * kSmallStride + 16 * (i >> 1) + 2 * r + (i & 1)] =
+            acc[i][j][h];
   __syncthreads();
-  // outputs: 40 consecutive rows of a column by consecutive threads
-  for (int q = threadIdx.x; q < wn * kSmallOut; q += 32 * kSmallWarps) {
-    const int w = q / kSmallOut, e = q % kSmallOut;
-    const int m = m0 + e % kSmallRows, n = n0 + w * kSmallCols + e / kSmallRows;
+  // outputs: 32 consecutive rows of a column by a warp
+  for (int q = warp; q < wn * kSmallCols; q += kSmallWarps) {
+    const int w = q / kSmallCols, e = (q % kSmallCols) * kSmallStride + lane;
+    const int m = m0 + lane, n = n0 + q;
     if (m >= g.M || n >= g.ncol) continue;
     double s = red[w][e];
     for (int z = 1; z < wk; ++z) s += red[w + z * wn][e];

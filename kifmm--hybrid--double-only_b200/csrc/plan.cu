@@ -255,18 +255,27 @@ kfmm_status upload(kfmm_plan* p, T** ptr, const std::vector<T>& h) {
 // Large tiles (160 x 64, kGemmRows x kGemmBN) when they give every SM its two
 // blocks and at least half of their rows are used (operators of at most 80 rows, NP
 // 3 and 4, take small tiles always: products of 4M points on the ellipsoid surface
-// 0.525 -> 0.510 ms); else small tiles, with the fewest column groups per CTA (the most
-// shares of K, up to the tuning's splitk_max) that leave at most two CTAs per SM.
+// 0.525 -> 0.506 ms).  Else small tiles, in the column groups per CTA (the other
+// warps share K, up to the tuning's splitk_max ways) with the least waves of two
+// CTAs per SM x (steps of K per warp + 4), 4 standing for a CTA's start and the
+// shares' sum.
 void choose_tiles(const kfmm_plan* p, GemmBatch& g) {
-  const int want = 2 * p->num_sms;
+  const long long resident = 2 * p->num_sms;
   g.wn = 0;
-  if (g.M > kGemmRows / 2 && g.chunks * ((g.ncol + kGemmBN - 1) / kGemmBN) >= want) return;
-  const int mt = (g.M + kSmallRows - 1) / kSmallRows;
-  auto ctas = [&](int wn) { return mt * ((g.ncol + kSmallCols * wn - 1) / (kSmallCols * wn)); };
-  g.wn = 1;
-  if (p->tune.splitk_max > 0)
-    while (kSmallWarps / g.wn > p->tune.splitk_max) g.wn *= 2;
-  while (g.wn < kSmallWarps && ctas(g.wn) > want) g.wn *= 2;
+  if (g.M > kGemmRows / 2 && g.chunks * ((g.ncol + kGemmBN - 1) / kGemmBN) >= resident) return;
+  const long long mt = (g.M + kSmallRows - 1) / kSmallRows;
+  long long best = -1;
+  for (int wn = 1; wn <= kSmallWarps; wn *= 2) {
+    const int shares = kSmallWarps / wn, cols = kSmallCols * wn;
+    if (p->tune.splitk_max > 0 && shares > std::max(1, p->tune.splitk_max)) continue;
+    const long long ctas = mt * ((g.ncol + cols - 1) / cols);
+    const long long steps = ((g.K + 7) / 8 + shares - 1) / shares;
+    const long long cost = (ctas + resident - 1) / resident * (steps + 4);
+    if (best < 0 || cost < best) {
+      best = cost;
+      g.wn = wn;
+    }
+  }
 }
 
 // Launches a kernel of the far field: with `chained`, its blocks may start before
