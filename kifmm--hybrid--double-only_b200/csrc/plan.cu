@@ -518,8 +518,7 @@ void add_part(std::vector<P2PJob>& jobs, const P2PJob& all, int from, int to) {
 void split_even(std::vector<P2PJob>& jobs, const P2PJob& all, int count, int rows) {
   const int full = (count + 31) / 32, parts = (full + rows - 1) / rows;
   for (int c = 0; c < parts; ++c)
-    add_part(jobs, all, 32 * (int)((long long)full * c / parts),
-             std::min(count, 32 * (int)((long long)full * (c + 1) / parts)));
+    add_part(jobs, all, 32 * (full * c / parts), std::min(count, 32 * (full * (c + 1) / parts)));
 }
 
 // One warp per job: parts of 32 * rows targets (rows: 0 for the automatic choice,
@@ -2224,13 +2223,26 @@ kfmm_status kfmm_batch_create(kfmm_plan* const* plans, int nplans, int nstreams,
   };
   if (!single) fork();
   kfmm_status st = KFMM_OK;
-  for (int i = 0; i < nplans && st == KFMM_OK; ++i) {
+  // Which branch takes which plan: a far field's time is mostly its launches' (each
+  // waits for the one before), so plans go, most launches first, to the branch with
+  // the fewest so far (32 solves, mixed 2.03 -> 1.92 ms, plain 3.91 -> 3.85 ms).
+  std::vector<int> order(nplans), branch(nplans, 0), load(nstreams, 0);
+  for (int i = 0; i < nplans; ++i) order[i] = i;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int c) {
+    return plans[a]->stats.launches > plans[c]->stats.launches;
+  });
+  for (int i : order) {
+    branch[i] = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+    load[branch[i]] += plans[i]->stats.launches;
+  }
+  for (int k = 0; k < nplans && st == KFMM_OK; ++k) {
+    const int i = order[k];
     const bool timing = plans[i]->timing;
     plans[i]->timing = false;
     // branches run side by side: waiting blocks of one would hold the others' slots
     // (32 solves 2.22 -> 2.35 ms)
     plans[i]->chained = false;
-    cudaStream_t on = single ? origin : b->streams[i % nstreams];
+    cudaStream_t on = single ? origin : b->streams[branch[i]];
     st = fused ? run_far_field(plans[i], on) : kfmm_run(plans[i], on);
     plans[i]->timing = timing;
     plans[i]->chained = true;
