@@ -129,15 +129,17 @@ kfmm_status kfmm_plan_create_with_operators(const kfmm_tree_desc* tree, int np,
 /* Kernel launch choices (no reference counterpart; the reference fixes its
  * thread-block sizes at compile time, fmm/cuda.cu:35-105).  0 in a field
  * keeps the plan's own choice.  The autotuner sweeps them.
- *   nf_blocks   mixed near field compiled for 5 or 6 resident blocks per SM
- *               (automatic: 5 when W-list surfaces carry > 1% of the pairs)
+ *   nf_blocks   mixed near field of one-warp jobs compiled for 5 or 6 resident
+ *               blocks per SM (automatic: 5 when W-list surfaces carry > 1% of
+ *               the pairs)
  *   job_rows    near-field jobs of at most 32 * job_rows targets, 1..6
- *               (automatic: 4 for mixed plans whose W lists carry > 1% of the
- *               pairs, else 6)
+ *               (automatic: one-warp jobs 4 for mixed plans whose W lists carry
+ *               > 1% of the pairs, else 6; team jobs, which plain plans and small
+ *               mixed ones use, at most 4, fewer where jobs are few)
  *   had_windows mixed Hadamard: sibling windows per warp of a CTA, 1..8
  *               (automatic: the shortest span in waves of one CTA per SM)
- *   splitk_max  level products: largest split-K factor (automatic:
- *               max(8, K / 64))
+ *   splitk_max  level products in small tiles: most warps that share K
+ *               (automatic: up to 8)
  *   had_tensor  mixed Hadamard on the tcgen05 tensor cores (TF32, three
  *               passes) for levels whose boxes are all present: 2 every
  *               complete level; 0 automatic and 1 none (the CUDA-core kernels,
@@ -197,12 +199,12 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* plan, void* stream); /* FFT, Hadamard, IF
 kfmm_status kfmm_xlist_calc(kfmm_plan* plan, void* stream); /* S2L part of X */
 kfmm_status kfmm_down_calc(kfmm_plan* plan, void* stream);  /* L2L */
 /* U list + W list + direct part of X + L2T, fused: each target's potential is
- * accumulated once, in registers, and written once (KFMM_MIXED plans: already
- * at the target's original index). */
+ * accumulated once, in registers, and written once, at the target's original
+ * index. */
 kfmm_status kfmm_ulist_calc(kfmm_plan* plan, void* stream);
-/* copy_trg_val (fmm/cuda.cu:2543-2565): potentials to original order on the
- * device (plain plans: a scatter; mixed plans: already there); pot_host (may
- * be NULL) additionally receives them (synchronous).
+/* copy_trg_val (fmm/cuda.cu:2543-2565): the near field has stored the potentials
+ * in original order on the device; pot_host (may be NULL) receives them
+ * (synchronous).
  * kfmm_get_potentials_device copies them to device memory and waits for
  * `stream`.  Both report KFMM_ERR_CUDA when a kernel of the last solve gave up
  * a bounded wait (the mixed V list's translation-tile copy); the flag is
