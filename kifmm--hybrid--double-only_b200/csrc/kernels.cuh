@@ -1023,6 +1023,8 @@ constexpr int kSmallStride = kSmallRows + 2;
 
 __global__ void __launch_bounds__(32 * kSmallWarps, 2) gemm_fp64_small_kernel(GemmArgs g, int wn) {
   __shared__ double red[kSmallWarps][kSmallCols * kSmallStride];  // [warp][col][row]
+  __shared__ int coff_s[kSmallCols * kSmallWarps];  // the epilogue's, read before the wait
+  __shared__ double alpha_s[kSmallCols * kSmallWarps];
   chain_release();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wk = kSmallWarps / wn, cg = warp % wn, ks = warp / wn;
@@ -1039,6 +1041,11 @@ __global__ void __launch_bounds__(32 * kSmallWarps, 2) gemm_fp64_small_kernel(Ge
 #pragma unroll
   for (int j = 0; j < 2; ++j)
     bp[j] = g.B + g.boff[min(g.ncol - 1, n0 + cg * kSmallCols + 8 * j + r)] + k0 + 2 * c;
+  for (int q = threadIdx.x; q < wn * kSmallCols; q += 32 * kSmallWarps) {
+    const bool in = n0 + q < g.ncol;
+    coff_s[q] = in ? g.coff[n0 + q] : 0;
+    alpha_s[q] = in && g.alpha ? g.alpha[n0 + q] : g.alpha_const;
+  }
   double acc[4][2][2];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
@@ -1085,17 +1092,28 @@ __global__ void __launch_bounds__(32 * kSmallWarps, 2) gemm_fp64_small_kernel(Ge
         red[warp][(8 * j + 2 * c + h) * kSmallStride + 16 * (i >> 1) + 2 * r + (i & 1)] =
             acc[i][j][h];
   __syncthreads();
-  // outputs: 32 consecutive rows of a column by a warp
-  for (int q = warp; q < wn * kSmallCols; q += kSmallWarps) {
-    const int w = q / kSmallCols, e = (q % kSmallCols) * kSmallStride + lane;
-    const int m = m0 + lane, n = n0 + q;
-    if (m >= g.M || n >= g.ncol) continue;
-    double s = red[w][e];
-    for (int z = 1; z < wk; ++z) s += red[w + z * wn][e];
-    const double a = g.alpha ? g.alpha[n] : g.alpha_const;
-    double* o = g.C + (size_t)g.coff[n] + m;
-    if (g.accumulate) *o += a * s;
-    else *o = a * s;
+  // outputs: 32 consecutive rows of a column by a warp, two columns at a time (the
+  // outputs to accumulate onto are read before either is written)
+  const int m = m0 + lane;
+  if (m >= g.M) return;
+  for (int q0 = warp; q0 < wn * kSmallCols; q0 += 2 * kSmallWarps) {
+    double* o[2];
+    double old[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int q = q0 + h * kSmallWarps;  // 16 wn columns: both exist
+      o[h] = n0 + q < g.ncol ? g.C + (size_t)coff_s[q] + m : nullptr;
+      old[h] = o[h] && g.accumulate ? *o[h] : 0.0;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (!o[h]) continue;
+      const int q = q0 + h * kSmallWarps, e = (q % kSmallCols) * kSmallStride + lane;
+      double s = red[q / kSmallCols][e];
+      for (int z = 1; z < wk; ++z) s += red[q / kSmallCols + z * wn][e];
+      s *= alpha_s[q];
+      *o[h] = g.accumulate ? old[h] + s : s;
+    }
   }
 }
 
