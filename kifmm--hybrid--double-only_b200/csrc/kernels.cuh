@@ -809,7 +809,8 @@ p2p_team_kernel(P2PArgs<kMixed> a) {
 }
 
 // The near fields of many plans in one launch (batched solves): job j is of the
-// plan whose arrays params[jobs[j].plan] describes.
+// plan whose arrays params[jobs[j].plan] describes.  32 solves of 4,096 to 262,144
+// points, mixed: 0.91 ms.
 template <bool kMixed>
 __global__ void __launch_bounds__(32 * kTeam, kMixed ? kTeamBlocksMixed : kTeamBlocksFp64)
 p2p_team_batch_kernel(const P2PArgs<kMixed>* params, const P2PJob* jobs) {
@@ -1018,6 +1019,9 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_fp64_dmma_kernel(GemmArg
 // more columns it is the L1's rate, so the fragments are read 16 bytes a lane: a
 // load of A holds rows 2r and 2r + 1 of one k (rows of two m8 tiles), a load of B
 // holds k 2c and 2c + 1 of one column (two k steps, of the even and the odd k).
+// Up and down products of a solve, split-K and a reduction pass -> 8-byte loads, 40
+// x 16 -> this: 20,011 points on a deep tree 346 -> 140 -> 94 us, 65,536 points NP 4
+// plain 141 -> 73 -> 52, 4M on the ellipsoid surface NP 4 678 -> 439 -> 303.
 constexpr int kSmallRows = 32, kSmallCols = 16, kSmallWarps = 8;
 constexpr int kSmallStride = kSmallRows + 2;
 
@@ -2234,7 +2238,9 @@ __global__ void gather_flags_kernel(int n, const int* const* flags, int* out) {
 // chunk prefetched into registers; a CTA's 16 warps are 16 / kSplit target tiles
 // times kSplit shares of the sources.  The shares are added in a fixed order, a
 // CTA's through shared memory and a cluster's through distributed shared memory,
-// so there is no scratch array, no atomic and one launch.
+// so there is no scratch array, no atomic and one launch.  1,000 targets x 1,048,576
+// sources: one thread per target 92.6 ms (8 blocks), this 1.14 ms (0.92e12 pairs/s
+// of 1.5e12; its 256 blocks leave 40 of 296 slots empty).
 constexpr int kDirectWarps = 16;
 constexpr int kDirectCluster = 8;
 

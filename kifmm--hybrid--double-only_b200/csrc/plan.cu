@@ -1111,26 +1111,29 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
       std::vector<int> pwin, pmem, swin, smem;
       // Present entries of a group's window but for the eight boxes of the group
       // itself, which are adjacent to every member, and the rows that hold any.
+      auto present = [&](int g, auto entry) {
+        const int* w = &win[(size_t)g * 216];
+        for (int z = 0, q = 0; z < 6; ++z)
+          for (int y = 0; y < 6; ++y)
+            for (int x = 0; x < 6; ++x, ++q) {
+              const bool own = (x == 2 || x == 3) && (y == 2 || y == 3) && (z == 2 || z == 3);
+              if (w[q] >= 0 && !own) entry(w[q], x, y, z);
+            }
+      };
       auto count = [&](int g, unsigned long long& rows) {
         int n = 0;
-        for (int q = 0; q < 216; ++q) {
-          const int x = q % 6, y = q / 6 % 6, z = q / 36;
-          const bool own = (x == 2 || x == 3) && (y == 2 || y == 3) && (z == 2 || z == 3);
-          if (win[(size_t)g * 216 + q] < 0 || own) continue;
+        present(g, [&](int, int, int y, int z) {
           ++n;
           rows |= 1ull << (y + 6 * z);
-        }
+        });
         return n;
       };
       std::vector<int> sp_ptr(1, 0), sp_mem;
       std::vector<int2> sp_ent;
       auto add_sparse = [&](int g) {
-        for (int q = 0; q < 216; ++q) {
-          const int x = q % 6, y = q / 6 % 6, z = q / 36;
-          const bool own = (x == 2 || x == 3) && (y == 2 || y == 3) && (z == 2 || z == 3);
-          if (win[(size_t)g * 216 + q] < 0 || own) continue;
-          sp_ent.push_back(make_int2(win[(size_t)g * 216 + q], (x + 1) + 7 * (y + 1) + 49 * (z + 1)));
-        }
+        present(g, [&](int node, int x, int y, int z) {
+          sp_ent.push_back(make_int2(node, (x + 1) + 7 * (y + 1) + 49 * (z + 1)));
+        });
         sp_ptr.push_back((int)sp_ent.size());
         sp_mem.insert(sp_mem.end(), &mem[(size_t)g * 8], &mem[(size_t)g * 8] + 8);
       };
@@ -1273,7 +1276,7 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
 
   // --- near field: U + W + direct X + L2T
   {
-    std::vector<P2PEntry> ent;
+    std::vector<P2PEntry> ent, list;
     // Pairs with W-list UE surfaces: where they carry more than 1% of the
     // pairs (clouds on surfaces), the mixed near field runs with 5 resident
     // blocks per SM and jobs of at most 4 rows (128 targets): measured on 4M
@@ -1354,23 +1357,23 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
       // entries without sources leave the list; the plain form's points carry
       // absolute coordinates, so ranges that touch become one (but not with the
       // leaf's own, whose pairs may coincide)
-      std::vector<P2PEntry> list(ent.begin() + e0, ent.end());
-      list.erase(std::remove_if(list.begin(), list.end(),
-                                [](const P2PEntry& q) { return q.count == 0; }),
-                 list.end());
+      list.clear();
+      for (size_t k = e0; k < ent.size(); ++k)
+        if (ent[k].count != 0 && (p->prec == KFMM_MIXED || ent[k].kind == 0)) list.push_back(ent[k]);
       if (p->prec != KFMM_MIXED) {
-        std::stable_sort(list.begin(), list.end(), [](const P2PEntry& a, const P2PEntry& b) {
-          return a.kind != b.kind ? a.kind < b.kind : a.kind == 0 && a.base < b.base;
-        });
+        std::sort(list.begin(), list.end(),
+                  [](const P2PEntry& a, const P2PEntry& b) { return a.base < b.base; });
         size_t m = 0;
         for (size_t k = 0; k < list.size(); ++k) {
-          if (m > 0 && list[k].kind == 0 && list[k].node != t && list[m - 1].node != t &&
+          if (m > 0 && list[k].node != t && list[m - 1].node != t &&
               list[m - 1].base + list[m - 1].count == list[k].base)
             list[m - 1].count += list[k].count;
           else
             list[m++] = list[k];
         }
         list.resize(m);
+        for (size_t k = e0; k < ent.size(); ++k)
+          if (ent[k].kind != 0) list.push_back(ent[k]);
       }
       ent.resize(e0);
       ent.insert(ent.end(), list.begin(), list.end());
