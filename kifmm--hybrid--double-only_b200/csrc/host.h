@@ -3,6 +3,7 @@
 // include/kifmm_b200.h.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -19,6 +20,19 @@ constexpr int kTrgTag = 2;  // LET_TRGNODE (fmm/input.h:13)
 constexpr double kOneOver4Pi = 1.0 / (4.0 * 3.14159265358979323846);
 
 void set_error(const std::string& msg);
+
+// `count` targets in the fewest parts of at most `rows` rows of 32 targets, the rows
+// spread evenly: how many parts, and where part c begins (c = parts: the end).  In
+// 64 bits: a tree splits on its sources alone, so one leaf may hold millions of
+// targets, and its rows times its parts pass 2^31 from 1.5 million on.
+inline int even_parts(int count, int rows) {
+  const long long full = (count + 31ll) / 32;
+  return (int)((full + rows - 1) / rows);
+}
+inline int even_part_begin(int count, int rows, int c) {
+  const long long full = (count + 31ll) / 32;
+  return (int)std::min((long long)count, 32 * (full * c / std::max(1, even_parts(count, rows))));
+}
 
 struct Tree {
   int num_src = 0, num_trg = 0;

@@ -518,9 +518,9 @@ void add_part(std::vector<P2PJob>& jobs, const P2PJob& all, int from, int to) {
 // A job's targets in parts of nearly equal numbers of 32-target rows, at most
 // `rows` each.
 void split_even(std::vector<P2PJob>& jobs, const P2PJob& all, int count, int rows) {
-  const int full = (count + 31) / 32, parts = (full + rows - 1) / rows;
+  const int parts = even_parts(count, rows);
   for (int c = 0; c < parts; ++c)
-    add_part(jobs, all, 32 * (full * c / parts), std::min(count, 32 * (full * (c + 1) / parts)));
+    add_part(jobs, all, even_part_begin(count, rows, c), even_part_begin(count, rows, c + 1));
 }
 
 // One warp per job: parts of 32 * rows targets (rows: 0 for the automatic choice,
