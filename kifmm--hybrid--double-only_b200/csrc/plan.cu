@@ -2203,16 +2203,19 @@ kfmm_status kfmm_batch_create(kfmm_plan* const* plans, int nplans, int nstreams,
         (e = cudaMemcpy(b->d_jobs, jobs.data(), jbytes, cudaMemcpyHostToDevice)) != cudaSuccess)
       return fail(e, "cudaMemcpy");
   }
+  cudaStream_t origin = b->streams[nstreams];
   {
     std::vector<const int*> flags(nplans);
     for (int i = 0; i < nplans; ++i) flags[i] = plans[i]->d_error;
-    const size_t fbytes = sizeof(int*) * nplans;
+    const size_t fbytes = sizeof(int*) * nplans, gbytes = sizeof(int) * nplans;
+    // d_gathered is read by a kfmm_batch_wait before the first launch too
     if ((e = cudaMalloc((void**)&b->d_flags, fbytes)) != cudaSuccess ||
-        (e = cudaMalloc((void**)&b->d_gathered, sizeof(int) * nplans)) != cudaSuccess ||
-        (e = cudaMemcpy(b->d_flags, flags.data(), fbytes, cudaMemcpyHostToDevice)) != cudaSuccess)
+        (e = cudaMalloc((void**)&b->d_gathered, gbytes)) != cudaSuccess ||
+        (e = cudaMemcpy(b->d_flags, flags.data(), fbytes, cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = cudaMemsetAsync(b->d_gathered, 0, gbytes, origin)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(origin)) != cudaSuccess)
       return fail(e, "error flags");
   }
-  cudaStream_t origin = b->streams[nstreams];
   if ((e = cudaStreamBeginCapture(origin, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
     return fail(e, "cudaStreamBeginCapture");
   // fork: every branch stream waits on the origin, then runs its plans

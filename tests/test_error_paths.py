@@ -69,3 +69,30 @@ def test_batch_wait_reports_timeout(K, cuda_ok):
     for p in plans:
         assert np.array_equal(p.potentials(), want)
     batch.close()
+
+
+@pytest.mark.gpu
+def test_batch_wait_before_a_launch(K, cuda_ok):
+    """Nothing was launched, so nothing ran out: a wait reports no error, whatever the
+    device memory the batch got held before."""
+    import ctypes
+    import torch
+    torch.cuda.init()
+    rt = ctypes.CDLL("libcudart.so.12")  # torch's, already loaded
+    pts, tree = _setup(K, n=3000)
+    plans = [K.Plan(tree, 4, K.MIXED) for _ in range(40)]
+    for p in plans:
+        p.set_points(pts)
+    torch.cuda.synchronize()
+    bufs = [ctypes.c_void_p() for _ in range(8192)]
+    for b in bufs:
+        assert rt.cudaMalloc(ctypes.byref(b), ctypes.c_size_t(512)) == 0
+        assert rt.cudaMemset(b, 1, ctypes.c_size_t(512)) == 0
+    assert rt.cudaDeviceSynchronize() == 0
+    for b in bufs:
+        assert rt.cudaFree(b) == 0
+    batch = K.Batch(plans, nstreams=2)
+    batch.wait()
+    batch.launch()
+    batch.wait()
+    batch.close()
