@@ -207,7 +207,7 @@ kfmm_status kfmm_ulist_calc(kfmm_plan* plan, void* stream);
  * (synchronous).
  * kfmm_get_potentials_device copies them to device memory and waits for
  * `stream`.  Both report KFMM_ERR_CUDA when a kernel of the last solve gave up
- * a bounded wait (the mixed V list's translation-tile copy); the flag is
+ * a bounded wait (the V list's translation-tile copy, in both forms); the flag is
  * cleared at the start of every solve, so a later solve that completes is
  * reported as KFMM_OK again.  (The reference exits on any CUDA error,
  * fmm/cuda.cu:19-30.) */

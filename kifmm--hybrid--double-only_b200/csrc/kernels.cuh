@@ -1621,7 +1621,8 @@ struct Had64Params {
   const double2* tile;  // [fb][343][32], zero for |delta|_inf <= 1 and f >= F
   const double2* spec;
   double2* effv;
-  int* error;  // set to 1 when the tile copy does not complete
+  int* error;            // set to 1 when the tile copy does not complete
+  long long wait_limit;  // tries of the tile-copy wait (kMbarSpinLimit by default)
 };
 
 template <int H>
@@ -1790,7 +1791,7 @@ __global__ void __launch_bounds__(kHad64Threads, 1) hadamard_fp64_kernel(Had64Pa
   __shared__ int mem[kHad64Warps][16];
   __shared__ __align__(8) unsigned long long bar;
   if (!had_load_tile<kHad64TileBytes>(p.tile + (size_t)blockIdx.y * 343 * kFB, had32_dyn, &bar,
-                                      p.error, kMbarSpinLimit))
+                                      p.error, p.wait_limit))
     return;
   const int chunk = blockIdx.x;
   const int single = chunk - p.pairs.chunks, sparse = single - p.singles.chunks;

@@ -1750,7 +1750,7 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
       }
     } else {
       Had64Params h{p->nn, p->pairs, p->singles, p->sparse, (const double2*)p->d_trans,
-                    (const double2*)p->spec, (double2*)p->effv, p->d_error};
+                    (const double2*)p->spec, (double2*)p->effv, p->d_error, p->wait_limit};
       const dim3 grid(p->pairs.chunks + p->singles.chunks + p->sparse.chunks, p->Fpad / kFB);
       launch_chained(p->chained, hadamard_fp64_kernel, grid, kHad64Threads, kHad64TileBytes, S(stream), h);
       KF_CHECK_LAUNCH("hadamard_fp64_kernel");

@@ -1,6 +1,6 @@
 """Error reporting of the kernels' bounded waits, driven without a fault.
 
-The mixed V list copies each frequency block's translation spectra into
+The V list, in both forms, copies each frequency block's translation spectra into
 shared memory with a bulk copy and waits on an mbarrier for a bounded number
 of tries; when the tries run out the kernel sets the plan's error flag and
 returns (after letting the copy land).  kfmm_set_wait_limit(plan, 0) makes
@@ -26,12 +26,17 @@ def test_set_wait_limit_rejects_null_plan(K):
     assert K.lib().kfmm_batch_wait(None, None) == 1
 
 
+FORMS = pytest.mark.parametrize("form", ["MIXED", "PLAIN_FP64"])
+
+
 @pytest.mark.gpu
-def test_wait_timeout_reported_then_cleared(K, cuda_ok):
+@FORMS
+def test_wait_timeout_reported_then_cleared(K, cuda_ok, form):
     import torch
+    prec = getattr(K, form)
     pts, tree = _setup(K)
-    want = K.Plan(tree, 4, K.MIXED).evaluate(pts)
-    plan = K.Plan(tree, 4, K.MIXED)
+    want = K.Plan(tree, 4, prec).evaluate(pts)
+    plan = K.Plan(tree, 4, prec)
     plan.set_wait_limit(0)
     with pytest.raises(K.KfmmError, match="bounded wait"):
         plan.evaluate(pts)
@@ -50,12 +55,14 @@ def test_wait_timeout_reported_then_cleared(K, cuda_ok):
 
 
 @pytest.mark.gpu
-def test_batch_wait_reports_timeout(K, cuda_ok):
+@FORMS
+def test_batch_wait_reports_timeout(K, cuda_ok, form):
+    prec = getattr(K, form)
     pts, tree = _setup(K, n=15000)
-    plans = [K.Plan(tree, 4, K.MIXED) for _ in range(2)]
+    plans = [K.Plan(tree, 4, prec) for _ in range(2)]
     for p in plans:
         p.set_points(pts)
-    want = K.Plan(tree, 4, K.MIXED).evaluate(pts)
+    want = K.Plan(tree, 4, prec).evaluate(pts)
     plans[1].set_wait_limit(0)
     batch = K.Batch(plans, nstreams=2)  # the limit is captured with the launch
     batch.launch()
