@@ -2196,10 +2196,28 @@ hadamard_fp32_sparse_kernel(HadSparse32Params p) {
 // (and, for mixed plans, a 16-byte record of FP32 offsets from the point's
 // leaf centre, leaf[i]) per store; gathering instead reads 8 bytes from four
 // random places per point (measured 0.21 ms against ... at 4M points).
+//
+// A coordinate beyond 2^510 is brought back to it, and a source that has one weighs
+// nothing: its r^2 would be infinite, where pair_rsqrt gives NaN without its guard,
+// while such a pair adds nothing (a source can be parked at infinity).
 __global__ void scatter_points_kernel(int n, const int* inv, const double* x, const double* y,
                                       const double* z, const double* w, double4* out) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-    out[inv[k]] = make_double4(x[k], y[k], z[k], w ? w[k] : 0.0);
+  constexpr double kFar = 0x1p510;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    double4 v = make_double4(x[k], y[k], z[k], w ? w[k] : 0.0);
+    bool far = false;
+    auto near = [&](double& c) {
+      if (fabs(c) > kFar) {
+        c = copysign(kFar, c);
+        far = true;
+      }
+    };
+    near(v.x);
+    near(v.y);
+    near(v.z);
+    if (far) v.w *= 0.0;  // NaN when the weight is not finite
+    out[inv[k]] = v;
+  }
 }
 
 // Mixed plans keep only the FP32 offsets (src4f); leaf[k]: source k's leaf.
