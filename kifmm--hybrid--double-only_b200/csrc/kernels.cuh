@@ -153,13 +153,17 @@ constexpr int kMaxSlots = 6;  // targets per lane: jobs hold up to 192 targets
 // Treatment of a Single Nonlinear Equation, 1970): with e = 1 - r2 y^2,
 // y (1 + e/2 + 3 e^2 / 8) leaves 5/16 e^3.  Five FP64 operations where rsqrt()
 // takes ten, and no branch, so several pairs' chains interleave; 1/(4 pi r) comes
-// out within 1.24 eps (tests/test_direct.py).  A pair is 12 FP64 operations
-// instead of 17: near field of 4M uniform points, NP 6, 15.6 -> 11.8 ms.
-// The caller starts its sum of squares from kTinyR2, so r2 is never subnormal or
-// zero.  kGuard: pairs whose r2 stays at that level (r = 0, as fmm/omp.cc:280
-// skips), is infinite or is not a number give 0, by an integer test on the high
-// word; it costs a tenth of the pair rate, so only sets that can hold such pairs
-// take it.
+// out within 1.24 eps as measured (tests/test_direct.py holds it to 3).  A pair is 12
+// FP64 operations instead of 17: near field of 4M uniform points, NP 6, 15.6 -> 11.8
+// ms.
+// kGuard, for sets that can hold r = 0 (a leaf's own sources, the direct sum): pairs
+// whose r2 is below the smallest normal number (r = 0, which fmm/omp.cc:280 skips;
+// r < 1.5e-154), infinite or not a number give 0, by an integer test on the high word.
+// It costs a tenth of the pair rate; rsqrt() in a branch for what lies below as well
+// costs the direct sum another 12% (1,144 -> 1,279 us) and the 100,003-point NP 8 solve
+// 6%.
+// Other sets start the sum of squares from kTinyR2, so that r2 is neither zero nor
+// subnormal there.
 constexpr double kTinyR2 = 0x1p-1020;
 template <bool kGuard>
 __device__ __forceinline__ double pair_rsqrt(double r2) {
@@ -168,7 +172,7 @@ __device__ __forceinline__ double pair_rsqrt(double r2) {
   const double e = fma(-r2, y * y, 1.0);
   y = fma(y * e, fma(e, 0.375, 0.5), y);
   if constexpr (kGuard) {
-    constexpr unsigned kLo = 0x00300001u;  // high word of 2^-1020, plus one
+    constexpr unsigned kLo = 0x00100000u;  // high word of the smallest normal number
     const bool ok = (unsigned)__double2hiint(r2) - kLo < 0x7ff00000u - kLo;
     y = ok ? y : 0.0;
   }
@@ -187,7 +191,7 @@ __device__ __forceinline__ void pairs_fp64(const double (&tx)[NS], const double 
 #pragma unroll
     for (int t = 0; t < NS; ++t) {
       const double dx = tx[t] - s.x, dy = ty[t] - s.y, dz = tz[t] - s.z;
-      const double r2 = fma(dz, dz, fma(dy, dy, fma(dx, dx, kTinyR2)));
+      const double r2 = fma(dz, dz, fma(dy, dy, kGuard ? dx * dx : fma(dx, dx, kTinyR2)));
       acc[t] = fma(s.w, pair_rsqrt<kGuard>(r2), acc[t]);
     }
   }

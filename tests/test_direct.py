@@ -39,6 +39,24 @@ def test_pair_term_accuracy(K, cuda_ok):
 
 
 @pytest.mark.gpu
+def test_tiny_distances(K, cuda_ok):
+    """The same bound down to the smallest r whose square is a normal number
+    (1.5e-154), in the direct sum and between the points of one leaf."""
+    rng = np.random.default_rng(2)
+    r = 10.0 ** rng.uniform(-153.7, -140, 20000)
+    x = r * rng.choice([-1.0, 1.0], r.size)
+    z, one = np.zeros_like(x), tuple(np.array([v]) for v in (0.0, 0.0, 0.0, 1.0))
+    ref = 1.0 / (4 * np.pi * r.astype(np.longdouble))
+    got = _direct(K, (x, z, z), one)
+    assert float(np.max(np.abs(got - ref) / ref)) <= 3 * EPS
+    pts = dict(zip(("sx", "sy", "sz", "den"), one), tx=x, ty=z, tz=z)
+    tree = K.Tree(*[pts[k] for k in ("sx", "sy", "sz", "tx", "ty", "tz")], 64)
+    assert tree.desc.num_nodes == 1
+    got = K.Plan(tree, 4, K.PLAIN_FP64).evaluate(pts)
+    assert float(np.max(np.abs(got - ref) / ref)) <= 3 * EPS
+
+
+@pytest.mark.gpu
 def test_skipped_pairs(K, cuda_ok):
     """Coincident points, sources at infinity and at NaN add nothing."""
     t = np.array([[0.25, 0.5], [0.5, 0.5], [-0.5, 0.125]])
