@@ -6,10 +6,10 @@ size) and the far field (grows with the number of boxes); the best leaf size
 depends on the point distribution, the point count, NP and the precision
 form.  At a given leaf size, the kernels' own shapes matter too: how many
 targets one near-field job holds (leaf chunking, `job_rows`), how many
-resident blocks per SM the mixed near-field kernel is compiled for
+resident blocks per SM the one-warp mixed near-field kernel is compiled for
 (`nf_blocks`, i.e. its register budget), how many sibling windows each warp
-of a mixed Hadamard CTA takes (`had_windows`) and how far the level products
-split their K dimension (`splitk_max`).
+of a mixed Hadamard CTA takes (`had_windows`) and how many warps may share the
+K dimension of a small level product (`splitk_max`).
 
 ``tune`` measures, on the device (CUDA events, kfmm_kernel_times), first
 every leaf-size candidate with the plan's automatic launch choices, then, at
@@ -31,11 +31,13 @@ import os
 CANDIDATES = (16, 32, 64, 128, 256, 512, 1024)
 # launch choices swept at the best leaf size, in this order; the first value
 # of each is the plan's automatic choice.  nf_blocks and had_windows only act
-# on mixed plans.
-KNOBS = (("job_rows", (0, 3, 4, 5, 6)),
+# on mixed plans; team near fields (plain plans, small mixed ones) ignore
+# nf_blocks and hold at most 4 rows a job; at most 8 warps share K, the automatic
+# limit.
+KNOBS = (("job_rows", (0, 1, 2, 3, 4, 5, 6)),
          ("nf_blocks", (0, 5, 6)),
          ("had_windows", (0, 2, 4, 6, 8)),
-         ("splitk_max", (0, 1, 2, 4, 16)))
+         ("splitk_max", (0, 1, 2, 4)))
 MIXED_ONLY = ("nf_blocks", "had_windows")
 KEEP_GAIN = 0.005
 
