@@ -133,7 +133,7 @@ struct kfmm_plan {
   float4* src4f = nullptr;
   int* d_src_leaf = nullptr;
   float4* ctrf = nullptr;
-  double *pot_leaf = nullptr, *pot_orig = nullptr;
+  double* pot_orig = nullptr;
   bool have_src = false, have_trg = false;
   // expansions
   double *uden = nullptr, *dchk = nullptr, *dden = nullptr, *chk_up = nullptr, *chk_m = nullptr;
@@ -842,7 +842,6 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
   KF_TRY(dalloc(p, &p->o_tz, p->nt));
   if (p->prec != KFMM_MIXED) KF_TRY(dalloc(p, &p->src4, p->ns));  // mixed kernels read src4f
   KF_TRY(dalloc(p, &p->trg4, p->nt));
-  KF_TRY(dalloc(p, &p->pot_leaf, p->nt));
   KF_TRY(dalloc(p, &p->pot_orig, p->nt));
   KF_TRY(dalloc(p, &p->uden, (size_t)nn * P));
   KF_TRY(dalloc(p, &p->dchk, (size_t)nn * P));
@@ -1383,9 +1382,11 @@ kfmm_status build_plan(kfmm_plan* p, const kfmm_tree_desc* d, const kfmm_operato
                                   d->trg_beg[t], 0, ns});
       p->stats.u_pairs += (double)d->trg_num[t] * ns;
     }
-    KF_TRY(upload(p, &p->nf_ent, ent));
-    if (p->prec == KFMM_MIXED) KF_TRY(upload(p, &p->nf_ids, ids_of(ent)));
     KF_TRY(build_nf_jobs(p));
+    // in the form that the jobs read (no change of the tuning turns team jobs into
+    // one-warp jobs or back)
+    if (p->prec == KFMM_MIXED && !p->nf_team) KF_TRY(upload(p, &p->nf_ids, ids_of(ent)));
+    else KF_TRY(upload(p, &p->nf_ent, ent));
   }
 
   fft_src_resident(p->np, p->prec == KFMM_MIXED);  // the occupancy query, before any capture
@@ -2056,7 +2057,7 @@ kfmm_status kfmm_read_array(kfmm_plan* p, int which, double* out, size_t count) 
     case 0: src = p->uden; avail = (size_t)p->nn * p->P; break;
     case 1: src = p->dchk; avail = (size_t)p->nn * p->P; break;
     case 2: src = p->dden; avail = (size_t)p->nn * p->P; break;
-    case 3: src = p->pot_leaf; avail = (size_t)p->nt; break;
+    case 3: src = p->pot_orig; avail = (size_t)p->nt; break;
     case 4:
       if (p->prec == KFMM_MIXED) {
         set_error("kfmm_read_array: spectra of a mixed plan are FP32");
@@ -2074,10 +2075,18 @@ kfmm_status kfmm_read_array(kfmm_plan* p, int which, double* out, size_t count) 
     return KFMM_ERR_INVALID;
   }
   KF_CUDA(cudaDeviceSynchronize());
-  if (which == 3) {  // leaf-order view of pot_orig
-    gather_pot_kernel<<<592, 256>>>(p->nt, p->d_trg_perm, p->pot_orig, p->pot_leaf);
-    KF_CHECK_LAUNCH("gather_pot_kernel");
-    KF_CUDA(cudaDeviceSynchronize());
+  if (which == 3 && count > 0) {  // leaf-order view of pot_orig
+    double* leaf = nullptr;
+    KF_CUDA(cudaMalloc((void**)&leaf, sizeof(double) * avail));
+    gather_pot_kernel<<<592, 256>>>(p->nt, p->d_trg_perm, p->pot_orig, leaf);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpy(out, leaf, count * sizeof(double), cudaMemcpyDeviceToHost);
+    cudaFree(leaf);
+    if (e != cudaSuccess) {
+      set_error(std::string("kfmm_read_array: ") + cudaGetErrorString(e));
+      return KFMM_ERR_CUDA;
+    }
+    return KFMM_OK;
   }
   KF_CUDA(cudaMemcpy(out, src, count * sizeof(double), cudaMemcpyDeviceToHost));
   return KFMM_OK;

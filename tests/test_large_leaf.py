@@ -99,3 +99,31 @@ def test_large_leaves_in_a_batch(K, cuda_ok, tuning):
     for plan, pts in zip(plans, cases):
         _check(plan.potentials(), *_reference(pts), False)
     batch.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["PLAIN_FP64", "MIXED"])
+def test_plan_memory_per_target(K, cuda_ok, form):
+    """A target costs 72 bytes of a plan: 24 of upload staging, 32 in leaf order, 8 of
+    permutations, 8 of potential.  Device memory comes in pages of 2 MiB, which rounds
+    these seven arrays up by 14 MiB at most; the rest of this plan (jobs 1.4 MB,
+    operators 3 MB, eight sources) takes five such pages at most.  Another 8 bytes
+    a target would be 30 MiB."""
+    import torch
+    prec = getattr(K, form)
+    small = K.generate_points(2000, "uniform", 0, 1)
+    tree = K.Tree(*[small[k] for k in ("sx", "sy", "sz", "tx", "ty", "tz")], 64)
+    K.Plan(tree, 4, prec).evaluate(small)  # modules loaded, flag slots allocated
+    nt = 4000000
+    pts = _leaf(nt)
+    tree = _tree(K, pts)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    plan = K.Plan(tree, 4, prec)
+    used = free - torch.cuda.mem_get_info()[0]
+    assert used <= 72 * nt + (24 << 20), used / nt
+    plan.set_points(pts)
+    plan.run()
+    got, leaf = plan.potentials(), plan.read(3, nt)
+    assert np.array_equal(leaf, got[tree.array("trg_perm")])
+    assert plan.read(3, 5).tolist() == leaf[:5].tolist()
