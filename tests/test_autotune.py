@@ -76,3 +76,47 @@ def test_set_tuning_in_place(K, cuda_ok, precision):
     got = plan.evaluate(pts)
     tol = 1e-9 if precision == "plain" else 1e-6
     assert np.linalg.norm(got - want) / np.linalg.norm(want) < tol
+
+
+def _many_leaves(K, seed=9):
+    """A cloud whose mixed near field runs one warp per job on any device of this
+    size: more target leaves than four times the warps that its SMs can hold."""
+    import torch
+    pts = K.generate_points(400000, "uniform", 0, seed)
+    tree = K.Tree(pts["sx"], pts["sy"], pts["sz"], pts["tx"], pts["ty"], pts["tz"], 12)
+    leaves = np.count_nonzero((tree.array("child") == -1) & (tree.array("trg_num") > 0))
+    assert leaves > 4 * 64 * torch.cuda.get_device_properties(0).multi_processor_count
+    return pts, tree
+
+
+@pytest.mark.gpu
+def test_set_tuning_of_one_warp_jobs(K, cuda_ok):
+    """The same for the one-warp near field, whose jobs job_rows re-chunks and whose
+    kernel nf_blocks chooses (the clouds above are small enough for team jobs)."""
+    pts, tree = _many_leaves(K)
+    plan = K.Plan(tree, 3, K.MIXED)
+    want = plan.evaluate(pts)
+    for cfg in ({"job_rows": 1}, {"job_rows": 3, "nf_blocks": 5}, {"job_rows": 6, "nf_blocks": 6},
+                {"nf_blocks": 5}, None):
+        plan.set_tuning(cfg)
+        assert np.array_equal(plan.evaluate(pts), want), cfg
+    plain = K.Plan(tree, 3, K.PLAIN_FP64).evaluate(pts)
+    # FP32 coordinates and pair terms, as on every uniform cloud
+    assert np.linalg.norm(want - plain) / np.linalg.norm(plain) < 1e-6
+
+
+@pytest.mark.gpu
+def test_one_warp_leaf_of_several_rows(K, cuda_ok):
+    """One-warp jobs of 1 to 6 rows: a single leaf of many targets (its 16,000 jobs are
+    more than four for each of the 24 x 148 warps that the kernel keeps resident)."""
+    rng = np.random.default_rng(4)
+    nt = 3000000 + 77
+    pts = {k: rng.uniform(-1, 1, 100) for k in ("sx", "sy", "sz")}
+    pts["den"] = rng.uniform(0, 1, 100)
+    pts.update({k: rng.uniform(-1, 1, nt) for k in ("tx", "ty", "tz")})
+    tree = K.Tree(*[pts[k] for k in ("sx", "sy", "sz", "tx", "ty", "tz")], 100, device=True)
+    plan = K.Plan(tree, 4, K.MIXED)
+    want = plan.evaluate(pts)
+    for rows in range(1, 7):
+        plan.set_tuning({"job_rows": rows})
+        assert np.array_equal(plan.evaluate(pts), want), rows

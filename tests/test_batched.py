@@ -46,6 +46,34 @@ def test_batched_graph_matches_single_runs(K, oracle_mod, cuda_ok, tmp_path):
     B.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["PLAIN_FP64", "MIXED"])
+@pytest.mark.parametrize("tuning", [None, {"job_rows": 2}])
+def test_batch_of_either_form_and_job_kind(K, cuda_ok, form, tuning):
+    """Batches whose near fields are team jobs (plain plans), and team jobs beside
+    one-warp jobs (a mixed plan of more target leaves than four times the device's
+    warps, between two small ones), bit for bit the single runs."""
+    import torch
+    prec = getattr(K, form)
+    plans, want = [], []
+    for n, dist, ppb, np_ in ((20000, "uniform", 40, 4), (400000, "uniform", 12, 3),
+                              (9000, "ellipsoidSurface", 24, 3)):
+        pts = K.generate_points(n, dist, 0, n)
+        tree = K.Tree(*[pts[k] for k in ("sx", "sy", "sz", "tx", "ty", "tz")], ppb)
+        leaves = np.count_nonzero((tree.array("child") == -1) & (tree.array("trg_num") > 0))
+        warps = 64 * torch.cuda.get_device_properties(0).multi_processor_count
+        assert (leaves > 4 * warps) == (n == 400000)
+        plans.append(K.Plan(tree, np_, prec, tuning=tuning))
+        want.append(plans[-1].evaluate(pts))
+    batch = K.Batch(plans, nstreams=2)
+    for _ in range(2):
+        batch.launch()
+        batch.wait()
+        for plan, w in zip(plans, want):
+            assert np.array_equal(plan.potentials(), w)
+    batch.close()
+
+
 def test_batch_rejects_bad_arguments(K):
     import ctypes
     h = ctypes.c_void_p()
