@@ -173,7 +173,7 @@ kfmm_status kfmm_plan_create_tuned(const kfmm_tree_desc* tree, int np, kfmm_prec
 /* New launch choices for an existing plan (NULL: all automatic): the
  * near-field jobs are re-chunked, the other choices are launch shapes; it
  * waits for the device first.  A batch that holds the plan must be created
- * again afterwards.  Only the split-K factor changes the order of any sum. */
+ * again afterwards.  Only splitk_max changes the order of any sum. */
 kfmm_status kfmm_plan_set_tuning(kfmm_plan* plan, const kfmm_tuning* tuning);
 kfmm_status kfmm_plan_destroy(kfmm_plan* plan);
 
@@ -282,9 +282,9 @@ kfmm_status kfmm_plan_stats(const kfmm_plan* plan, kfmm_stats* stats);
 kfmm_status kfmm_enable_timing(kfmm_plan* plan, int enable);
 kfmm_status kfmm_phase_times(const kfmm_plan* plan, float* ms6);
 /* Finer split of the same run (ms): [S2M pair sums, upward level products
- * (UC2UE, M2M; includes zeroing the downward check potentials), forward FFT,
+ * (UC2UE, M2M), forward FFT (also zeroes the downward check potentials),
  * Hadamard, inverse FFT, S2L, downward level products (L2L), near field,
- * copy]. */
+ * copy (nothing: the near field stores original order)]. */
 kfmm_status kfmm_kernel_times(const kfmm_plan* plan, float* ms9);
 
 /* Allocation-free S2M for a batch of leaves; it has no counterpart in the

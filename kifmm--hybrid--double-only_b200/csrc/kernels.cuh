@@ -32,9 +32,10 @@ __device__ __forceinline__ unsigned smem_addr(const void* p) {
 // that kernel is done (chain_wait).  What lies before the wait reads only what the
 // plan's creation wrote.  Every block of every such kernel waits, so the order
 // holds from end to end; launched in the ordinary way both are without effect.
-// 20,011 points on a deep tree (34 such launches) 281 -> 217 us, 4,096 points 108
-// -> 92 us.  The pair kernels are launched in the ordinary way: their waiting
-// blocks took the slots of what ran before them (65,536 points 358 -> 417 us).
+// Device time of a solve, ordinary launches -> these: 20,011 points on a deep tree
+// (32 such launches) 221 -> 162 us, 4,096 points 95 -> 78, 65,536 333 -> 309.  The
+// pair kernels are launched in the ordinary way: their waiting blocks took the slots
+// of what ran before them (65,536 points 358 -> 417 us when that was tried).
 __device__ __forceinline__ void chain_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -798,7 +799,7 @@ p2p_warp_kernel(P2PArgs<kMixed> a, int njobs, int* next_job) {
 // job order, largest first.  A job's time is a quarter of what one warp takes, so
 // near fields with few jobs per resident warp neither wait for the longest of
 // them nor leave warps idle: 65,536 points NP 4 plain 0.95 -> 0.16 ms, 1M points
-// NP 6 mixed 2.17 -> 1.92 ms.  Resident blocks asked of ptxas: plain 4 (119
+// NP 6 mixed 2.17 -> 1.94 ms.  Resident blocks asked of ptxas: plain 4 (119
 // registers; 5 and 6 measured 2% slower at 4M points), mixed 8 (64 registers; 5 to
 // 7 measured 1-5% slower at 1M and 4M).
 constexpr int kTeamBlocksFp64 = 4, kTeamBlocksMixed = 8;
@@ -2199,7 +2200,7 @@ hadamard_fp32_sparse_kernel(HadSparse32Params p) {
 // coalesced) goes to leaf-order position inv[k], one full 32-byte record
 // (and, for mixed plans, a 16-byte record of FP32 offsets from the point's
 // leaf centre, leaf[i]) per store; gathering instead reads 8 bytes from four
-// random places per point (measured 0.21 ms against ... at 4M points).
+// random places per point.
 //
 // A coordinate beyond 2^510 is brought back to it, and a source that has one weighs
 // nothing: its r^2 would be infinite, where pair_rsqrt gives NaN without its guard,

@@ -10,9 +10,9 @@
 //   down  : L2L per level, shallowest first (fmm/cuda.cu:1981-2045)
 //   ulist : one fused kernel per target chunk: U list, W list, direct X list,
 //           and L2T (fmm/cuda.cu:604-663, 2070-2197, 1804-1872)
-//   copy  : potentials back to original order (fmm/cuda.cu:2543-2565)
-// The reference adds U/W/X/L2T contributions into one array in four passes;
-// here each target's potential is summed once in registers and written once.
+// The reference adds U/W/X/L2T contributions into one array in four passes and
+// copies it back to original order in a fifth (fmm/cuda.cu:2543-2565); here each
+// target's potential is summed once in registers and written once, in place.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -301,8 +301,9 @@ void count_launches(kfmm_plan* p) {
   p->stats.tensor_levels = p->n_tc_levels;
   p->stats.host_pairs = p->host_pairs;
   p->stats.launches = (p->n_s2m > 0) + (int)p->up_gemms.size() + (p->n_fft > 0) +
-                      (p->prec == KFMM_MIXED ? (p->pairs.nwin > 0) + (p->singles.nwin > 0) + (p->sparse.n > 0)
-                                             : (p->n_groups > 0)) +
+                      (p->prec == KFMM_MIXED
+                           ? (p->pairs.nwin > 0) + (p->singles.nwin > 0) + (p->sparse.n > 0)
+                           : (p->n_groups > 0)) +
                       (p->n_tc_levels > 0) + (p->n_ifft > 0) + (p->n_s2l > 0) +
                       (int)p->down_gemms.size() + (p->n_nf > 0);
 }
@@ -341,7 +342,8 @@ kfmm_status add_gemm(kfmm_plan* p, std::vector<GemmBatch>& out, const double* A,
 
 kfmm_status launch_gemms(const kfmm_plan* p, const std::vector<GemmBatch>& gs, cudaStream_t st) {
   for (const GemmBatch& b : gs) {
-    GemmArgs a{b.A, b.M, b.K, b.B, b.boff, b.C, b.coff, b.alpha, b.alpha_const, b.ncol, b.accumulate};
+    GemmArgs a{b.A,    b.M,     b.K,           b.B,    b.boff,      b.C,
+               b.coff, b.alpha, b.alpha_const, b.ncol, b.accumulate};
     if (b.wn) {
       const int cols = kSmallCols * b.wn;
       dim3 grid((b.M + kSmallRows - 1) / kSmallRows, (b.ncol + cols - 1) / cols);
@@ -350,10 +352,8 @@ kfmm_status launch_gemms(const kfmm_plan* p, const std::vector<GemmBatch>& gs, c
       continue;
     }
     dim3 grid(b.chunks, (b.ncol + kGemmBN - 1) / kGemmBN);
-    if (b.accumulate)
-      launch_chained(p->chained, gemm_fp64_dmma_kernel<true>, grid, kGemmThreads, kGemmSmemBytes, st, a, b.mrows);
-    else
-      launch_chained(p->chained, gemm_fp64_dmma_kernel<false>, grid, kGemmThreads, kGemmSmemBytes, st, a, b.mrows);
+    auto kern = b.accumulate ? gemm_fp64_dmma_kernel<true> : gemm_fp64_dmma_kernel<false>;
+    launch_chained(p->chained, kern, grid, kGemmThreads, kGemmSmemBytes, st, a, b.mrows);
     KF_CHECK_LAUNCH("gemm_fp64_dmma_kernel");
   }
   return KFMM_OK;
@@ -485,11 +485,11 @@ constexpr double kCostClassWidth = 1.05;  // cost ratio spanned by one job-order
 
 // Order of P2P jobs: largest first by cost class (target slots x sources over
 // copies, in classes 5% wide; counting the copies: near field of 1M points, NP 6,
-// mixed 1.96 -> 1.94 ms, 100,003 points, NP 8, plain 377 -> 369 us); within a class the jobs keep their tree order, so warps
-// working at the same time read neighbouring leaves' sources and the L2 cache
-// serves the repeats (4M points, NP=6 uniform / NP=4 ellipsoid surface, mixed near
-// field: classes 25% wide 4.44 / 2.32 ms, 12% 4.39 / 2.28, 5% 4.39 / 2.27, 100%
-// 4.48 / 2.50).
+// mixed 1.96 -> 1.94 ms, 100,003 points, NP 8, plain 377 -> 369 us); within a class
+// the jobs keep their tree order, so warps working at the same time read
+// neighbouring leaves' sources and the L2 cache serves the repeats (4M points, NP=6
+// uniform / NP=4 ellipsoid surface, mixed near field: classes 25% wide 4.44 / 2.32
+// ms, 12% 4.39 / 2.28, 5% 4.39 / 2.27, 100% 4.48 / 2.50).
 void order_jobs(std::vector<P2PJob>& jobs) {
   std::vector<std::pair<double, int>> key(jobs.size());
   for (size_t j = 0; j < jobs.size(); ++j) {
@@ -531,16 +531,17 @@ void split_even(std::vector<P2PJob>& jobs, const P2PJob& all, int count, int row
 void add_row_jobs(const kfmm_plan* p, std::vector<P2PJob>& jobs, int rows) {
   if (rows == 0) rows = p->prec == KFMM_MIXED && p->nf_w_heavy ? 4 : kMaxSlots;
   for (const P2PJob& L : p->nf_leaf)
-    for (int c = 0; c < L.tcnt; c += 32 * rows) add_part(jobs, L, c, std::min(L.tcnt, c + 32 * rows));
+    for (int c = 0; c < L.tcnt; c += 32 * rows)
+      add_part(jobs, L, c, std::min(L.tcnt, c + 32 * rows));
 }
 
-// Team jobs: at most `rows` rows of 32 targets.  A
-// leaf's last row of at most 16 targets becomes a job of its own, whose warps
-// hold 2 or 4 copies of the targets and share the sources among them, when the
-// lists' entries are long enough to pay for walking them again (64 sources on
-// average; plain near field of 4M uniform points 12.25 -> 11.53 ms; with short
-// entries it loses: 4M points on the ellipsoid surface, mixed, 2.38 -> 2.54 ms).
-// Copies change the order of a target's sum, so they depend on the leaf alone.
+// Team jobs: at most `rows` rows of 32 targets.  A leaf's last row of at most 16
+// targets becomes a job of its own, whose warps hold 2 or 4 copies of the targets
+// and share the sources among them, when the lists' entries are long enough to pay
+// for walking them again (64 sources on average; plain near field of 4M uniform
+// points 12.25 -> 11.53 ms; with short entries it loses: 4M points on the ellipsoid
+// surface, mixed, 2.38 -> 2.54 ms).  Copies change the order of a target's sum, so
+// they depend on the leaf alone.
 void add_team_jobs(const kfmm_plan* p, std::vector<P2PJob>& jobs, int rows) {
   auto copies = [](int targets) { return targets <= 8 ? 4 : targets <= 16 ? 2 : 1; };
   for (const P2PJob& L : p->nf_leaf) {
@@ -555,7 +556,7 @@ void add_team_jobs(const kfmm_plan* p, std::vector<P2PJob>& jobs, int rows) {
 // Whether a near field of `row_jobs` one-warp jobs runs as teams instead.  Plain
 // form: always (also at 13 jobs per resident warp, 4M uniform points, 11.97 ->
 // 11.28 ms).  Mixed form: below 4 jobs per resident warp (1M points NP 6, 2.3 jobs
-// per warp: 2.17 -> 1.92 ms; at 9, 4M points, 4.38 against 4.37 ms; at 22, the
+// per warp: 2.17 -> 1.94 ms; at 9, 4M points, 4.38 against 4.37 ms; at 22, the
 // ellipsoid surface, 2.26 against 2.38 ms: the longer walk's cost shows on short
 // entries).
 bool use_teams(bool mixed, size_t row_jobs, int p2p_grid) {
@@ -1721,7 +1722,8 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
         HadPairParams h{p->nn, q.nwin, q.win_per_block, q.win, q.members, q.rows,
                         (const float2*)p->d_trans, (const float2*)p->spec, (float2*)p->effv,
                         p->d_error, p->wait_limit};
-        launch_chained(p->chained, hadamard_fp32_pair_kernel, dim3(q.chunks, nfb), kHadPairThreads, kHadPairSmemBytes, S(stream), h);
+        launch_chained(p->chained, hadamard_fp32_pair_kernel, dim3(q.chunks, nfb),
+                       kHadPairThreads, kHadPairSmemBytes, S(stream), h);
         KF_CHECK_LAUNCH("hadamard_fp32_pair_kernel");
       }
       if (p->singles.nwin) {
@@ -1729,13 +1731,15 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
         Had32Params h{p->nn, q.nwin, q.win_per_block, q.win, q.members, q.rows,
                       (const float2*)p->d_trans, (const float2*)p->spec, (float2*)p->effv,
                       p->d_error, p->wait_limit};
-        launch_chained(p->chained, hadamard_fp32_kernel, dim3(q.chunks, nfb), kHad32Threads, kHad32TileBytes, S(stream), h);
+        launch_chained(p->chained, hadamard_fp32_kernel, dim3(q.chunks, nfb), kHad32Threads,
+                       kHad32TileBytes, S(stream), h);
         KF_CHECK_LAUNCH("hadamard_fp32_kernel");
       }
       if (p->sparse.n) {
         HadSparse32Params h{p->nn, p->sparse, (const float2*)p->d_trans, (const float2*)p->spec,
                             (float2*)p->effv, p->d_error, p->wait_limit};
-        launch_chained(p->chained, hadamard_fp32_sparse_kernel, dim3(p->sparse.chunks, nfb), kHadSparseThreads, kHad32TileBytes, S(stream), h);
+        launch_chained(p->chained, hadamard_fp32_sparse_kernel, dim3(p->sparse.chunks, nfb),
+                       kHadSparseThreads, kHad32TileBytes, S(stream), h);
         KF_CHECK_LAUNCH("hadamard_fp32_sparse_kernel");
       }
       if (p->n_tc_levels) {
@@ -1753,7 +1757,8 @@ kfmm_status kfmm_vlist_calc(kfmm_plan* p, void* stream) {
       Had64Params h{p->nn, p->pairs, p->singles, p->sparse, (const double2*)p->d_trans,
                     (const double2*)p->spec, (double2*)p->effv, p->d_error, p->wait_limit};
       const dim3 grid(p->pairs.chunks + p->singles.chunks + p->sparse.chunks, p->Fpad / kFB);
-      launch_chained(p->chained, hadamard_fp64_kernel, grid, kHad64Threads, kHad64TileBytes, S(stream), h);
+      launch_chained(p->chained, hadamard_fp64_kernel, grid, kHad64Threads, kHad64TileBytes,
+                     S(stream), h);
       KF_CHECK_LAUNCH("hadamard_fp64_kernel");
     }
   }

@@ -39,7 +39,8 @@ def test_split_covers_every_target_once(split, count, rows):
         full = -(-count // 32)
         assert lo == 32 * (full * c // parts) and hi == min(count, 32 * (full * (c + 1) // parts))
         assert 0 < hi - lo <= 32 * rows
-    assert parts == 0 or (split.begin(count, rows, 0), split.begin(count, rows, parts)) == (0, count)
+    ends = split.begin(count, rows, 0), split.begin(count, rows, parts)
+    assert parts == 0 or ends == (0, count)
 
 
 def _leaf(nt):
@@ -54,7 +55,7 @@ def _reference(pts):
     """The direct sum and the closest pair."""
     out, near = np.zeros(len(pts["tx"])), np.inf
     for j in range(8):
-        r = np.sqrt(sum((pts[t] - pts[s][j]) ** 2 for t, s in (("tx", "sx"), ("ty", "sy"), ("tz", "sz"))))
+        r = np.sqrt(sum((pts["t" + c] - pts["s" + c][j]) ** 2 for c in "xyz"))
         near = min(near, r.min())
         out += pts["den"][j] / r
     return out / (4 * np.pi), near
