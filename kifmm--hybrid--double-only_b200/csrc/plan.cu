@@ -70,28 +70,22 @@ struct GemmBatch {
 // copy to pageable memory costs a staging pass and a wait of its own (about 8 us of
 // every solve handed back), and a pinned allocation per plan costs more than
 // creating a small plan (4,096 points: 3 -> 13 ms), so plans share one page of
-// slots, allocated with the first plan and kept; a plan that finds none free reads
-// its flags through pageable memory.  A page lost to a device reset is replaced.
+// slots; a plan that finds none free reads its flags through pageable memory.  The
+// page is the library's own memory, registered with the first plan: the
+// registration belongs to one context and goes with it (a device reset), but the
+// slots of plans on other devices stay valid memory, pageable until the next plan
+// registers the page again.
 class FlagSlots {
  public:
+  FlagSlots() {
+    for (int i = kSlots - 1; i >= 0; --i) free_.push_back(slots_ + 2 * i);
+  }
   int* take() {
     std::lock_guard<std::mutex> lock(mu_);
     cudaPointerAttributes at{};
-    if (base_ &&
-        (cudaPointerGetAttributes(&at, base_) != cudaSuccess || at.type != cudaMemoryTypeHost)) {
-      cudaGetLastError();
-      base_ = nullptr;
-    }
-    if (!base_) {
-      void* v = nullptr;
-      if (cudaHostAlloc(&v, sizeof(int) * 2 * kSlots, cudaHostAllocPortable) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-      }
-      base_ = (int*)v;
-      free_.clear();
-      for (int i = kSlots - 1; i >= 0; --i) free_.push_back(base_ + 2 * i);
-    }
+    if (cudaPointerGetAttributes(&at, slots_) != cudaSuccess || at.type != cudaMemoryTypeHost)
+      cudaHostRegister(slots_, sizeof(slots_), cudaHostRegisterPortable);
+    cudaGetLastError();
     if (free_.empty()) return nullptr;
     int* s = free_.back();
     free_.pop_back();
@@ -99,14 +93,14 @@ class FlagSlots {
   }
   void give(int* s) {
     std::lock_guard<std::mutex> lock(mu_);
-    if (s && base_ && s >= base_ && s < base_ + 2 * kSlots) free_.push_back(s);
+    if (s) free_.push_back(s);
   }
 
  private:
-  static constexpr int kSlots = 512;  // 4 KiB
+  static constexpr int kSlots = 512;
   std::mutex mu_;
-  int* base_ = nullptr;
   std::vector<int*> free_;
+  alignas(4096) int slots_[2 * kSlots] = {};  // one page
 };
 static FlagSlots g_flag_slots;
 

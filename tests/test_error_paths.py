@@ -11,8 +11,14 @@ potentials as an untouched plan (the flag is cleared at the start of each
 solve).  The reference has no such path: it exits on any CUDA error
 (fmm/cuda.cu:19-30).
 """
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def _setup(K, n=20000, ppb=32, np_=4):
@@ -103,3 +109,52 @@ def test_batch_wait_before_a_launch(K, cuda_ok):
     batch.launch()
     batch.wait()
     batch.close()
+
+
+# The first plan of the process lives in a context of its own, which ends while a plan
+# of the device's primary context is in use (as when one of two devices is reset).
+ENDED_CONTEXT = """
+import ctypes
+import sys
+sys.path.insert(0, sys.argv[1])
+import numpy as np
+import __graft_entry__
+K = __graft_entry__.load_package()
+pts = K.generate_points(5000, "uniform", 0, 26)
+tree = K.Tree(*[pts[k] for k in ("sx", "sy", "sz", "tx", "ty", "tz")], 32)
+cu = ctypes.CDLL("libcuda.so.1")
+def ok(rc):
+    assert rc == 0, rc
+dev, ctx = ctypes.c_int(), ctypes.c_void_p()
+ok(cu.cuInit(0))
+ok(cu.cuDeviceGet(ctypes.byref(dev), 0))
+ok(cu.cuCtxCreate_v2(ctypes.byref(ctx), 0, dev))
+first = K.Plan(tree, 4, K.MIXED)
+want = first.evaluate(pts)
+ok(cu.cuCtxPopCurrent_v2(ctypes.byref(ctypes.c_void_p())))
+plan = K.Plan(tree, 4, K.MIXED)
+assert np.array_equal(plan.evaluate(pts), want)
+ok(cu.cuCtxPushCurrent_v2(ctx))
+first.close()
+ok(cu.cuCtxPopCurrent_v2(ctypes.byref(ctypes.c_void_p())))
+ok(cu.cuCtxDestroy_v2(ctx))
+assert np.array_equal(plan.evaluate(pts), want)
+later = K.Plan(tree, 4, K.MIXED)
+for p in (later, plan):
+    p.set_wait_limit(0)
+    try:
+        p.evaluate(pts)
+        raise SystemExit("the flag did not arrive")
+    except K.KfmmError as e:
+        assert "bounded wait" in str(e)
+    p.set_wait_limit(-1)
+    assert np.array_equal(p.evaluate(pts), want)
+print("done")
+"""
+
+
+@pytest.mark.gpu
+def test_flags_outlive_the_first_plans_context(cuda_ok):
+    r = subprocess.run([sys.executable, "-c", ENDED_CONTEXT, ROOT], capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and "done" in r.stdout, r.stdout + r.stderr
